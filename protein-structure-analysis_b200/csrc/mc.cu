@@ -363,8 +363,17 @@ __global__ void __launch_bounds__(NT, 512 / NT) mc_kernel(MoveCtx C, MCConfigDev
     __shared__ int64_t ssm[33];
     const Team<CL> T;
     const int s = cfg.sys_order ? cfg.sys_order[blockIdx.x / CL] : (int)(blockIdx.x / CL);
-    if (threadIdx.x == 0) S = states[s];
-    __syncthreads();
+    if (threadIdx.x == 0) {
+        S = states[s];
+        // Whoever used the scratch last (another runner on this batch, a
+        // single-move call) may have left the counters of its final parity,
+        // which only its own next proposal would clear.
+        if (T.rank == 0) {
+            for (int k = 0; k < QUEUE_PER_SYS; ++k) C.w.queue[QUEUE_PER_SYS * s + k] = 0;
+            C.w.drift[2 * s] = C.w.drift[2 * s + 1] = 0;
+        }
+    }
+    T.sync();
     bool rows_ok = system_within_skin(C, s);
     if (threadIdx.x == 0 && !rows_ok && C.nl.ref_xyz && S.step < step_limit) S.need_rebuild = 1;
     __syncthreads();

@@ -273,3 +273,37 @@ def test_spec_wait_runs_out_and_reports():
     assert int(status.item()) & _lib.ST_SPEC_ABORT
     assert time.perf_counter() - t0 < 30.0
     assert float(torch.ones(4, device="cuda").sum()) == 4.0  # the context still works
+
+
+@pytest.mark.parametrize("cluster", [1, 8])
+@pytest.mark.parametrize("before", ["odd", "even", "single-move"])
+def test_second_runner_on_a_used_batch(cluster, before):
+    """A new runner starts on clean counters whatever the batch's scratch was
+    last used for (an odd or even number of proposals, a single-move call):
+    the chain is a fresh batch's, bit for bit."""
+    from protein_physics_b200.device import DeviceBatch
+    from protein_physics_b200.mc import MCRunner
+    g, F = _setup("insulin")
+
+    def chain(b):
+        st = MCRunner(b, 0.6, 9, cluster_size=cluster, spec_teams=1).run_to(12)
+        return b.coords(0), int(st["n_accepted"][0]), float(st["energy"][0])
+
+    def fresh():
+        return DeviceBatch([(g["xyz"], g["q"], g["r"], g["eps"], F)])
+
+    b = fresh()
+    if before == "single-move":
+        b.move_dE([0], [3], [[0.1, 0.0]])
+    else:
+        R = MCRunner(b, 0.6, 4, cluster_size=cluster, spec_teams=1)
+        n = 0
+        while n < 9 and (n == 0 or int(R.state()["n_proposed"][0]) % 2 != (before == "odd")):
+            n += 1
+            R.run_to(n)
+        assert int(R.state()["n_proposed"][0]) % 2 == (before == "odd")
+        b.load_coords(g["xyz"])
+    x, acc, e = chain(b)
+    x0, acc0, e0 = chain(fresh())
+    assert acc == acc0 and e == e0
+    np.testing.assert_array_equal(x, x0)
