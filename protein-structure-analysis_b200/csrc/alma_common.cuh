@@ -35,6 +35,26 @@ void alma_count_launches(int n);
     } while (0)
 #define ALMA_LAUNCH_CHECK(what) ALMA_LAUNCH_CHECK_N(what, 1)
 
+// Launches kfn on a grid of thread-block clusters of `cluster` CTAs (1-8,
+// the portable sizes) with smem bytes of dynamic shared memory each.
+template <typename... P, typename... A>
+inline cudaError_t alma_launch_cluster(void (*kfn)(P...), unsigned grid, unsigned block, unsigned cluster,
+                                       size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(block, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kfn, static_cast<P>(args)...);
+}
+
 // ---------------------------------------------------------------------------
 // energy model (physics_engine.cpp:181-196, :2007-2011, :2148-2164)
 // ---------------------------------------------------------------------------
@@ -372,6 +392,28 @@ __device__ __forceinline__ int sys_of_atom(const int32_t *atom_off, int nsys, in
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (atom_off[mid] <= i) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// Tiles of T atoms that do not cross systems: system s owns the tile slots
+// from atom_off[s] / T + s on (at least ceil(n_s / T) of them), so natoms / T
+// + nsys slots cover every batch and a slot's system is a binary search.  The
+// tiling of a system depends on its own atoms only: sums taken by tile are
+// the same for a chain alone and in a batch.
+template <int T>
+__host__ __device__ __forceinline__ int tile_slots(int natoms, int nsys) { return natoms / T + nsys; }
+
+template <int T>
+__device__ __forceinline__ int tile_base(const int32_t *atom_off, int s) { return atom_off[s] / T + s; }
+
+template <int T>
+__device__ __forceinline__ int sys_of_tile(const int32_t *atom_off, int nsys, int slot) {
+    int lo = 0, hi = nsys - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tile_base<T>(atom_off, mid) <= slot) lo = mid;
         else hi = mid - 1;
     }
     return lo;

@@ -14,6 +14,8 @@ descent minimisation, MALA and the autograd wrapper (through the C ABI).
     from the oracle energy and the autograd torsion gradient at the
     proposal; runs are reproducible from the seed.
 """
+import os
+
 import numpy as np
 import pytest
 
@@ -263,3 +265,39 @@ def test_mala_graph_replay_equals_eager():
     assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
     for k in ("energy", "n_accepted", "n_proposed", "step", "scale"):
         assert np.array_equal(out[0][0][k], out[1][0][k]), k
+
+
+@pytest.mark.parametrize("residues", [(16, 5, 31), (170,), (300,), (620,)])
+def test_torsion_tiles_and_clusters(residues):
+    """Chains whose atoms end inside, at and past a tile of the prefix sums,
+    and whose bond counts take each cluster size: the torsion gradient of a
+    random field and the all-bond move against numpy."""
+    from conftest import ROOT
+    from protein_physics_b200.device import DeviceBatch
+    from protein_physics_b200.topology import BondTopology, flatten
+    from protein_physics_b200.torsion import TorsionSpace
+    w = np.load(os.path.join(ROOT, "workloads", "c4_globule_1000res.npz"), allow_pickle=False)
+    ridx, systems, topos = w["res_idx"], [], []
+    for k, n in enumerate(residues):
+        r0 = 40 * k
+        a, b_ = np.searchsorted(ridx, [r0, r0 + n])
+        T = BondTopology()
+        T.build([str(v) for v in w["resnames"][a:b_]], [str(v) for v in w["atomnames"][a:b_]],
+                [int(v) - r0 for v in ridx[a:b_]])
+        topos.append(T)
+        systems.append((w["xyz"][a:b_].astype(np.float64), w["charge"][a:b_], w["radius"][a:b_], w["epsilon"][a:b_],
+                        flatten(T)))
+    b = DeviceBatch(systems)
+    ts = TorsionSpace(b)
+    rng = np.random.default_rng(7)
+    grad = np.zeros((b.natoms, 4))
+    grad[:, :3] = rng.normal(0, 10.0, (b.natoms, 3))
+    gth = ts.gtheta(torch.as_tensor(grad, device="cuda")).cpu().numpy()
+    delta = rng.normal(0, 0.05, ts.nrb)
+    ts.apply(torch.as_tensor(delta, device="cuda"))
+    for s, (x, _, _, _, flat) in enumerate(systems):
+        k0, k1, a0 = b.rb_off_h[s], b.rb_off_h[s + 1], b.atom_off_h[s]
+        ref = _autograd_gtheta(x, grad[a0:a0 + flat.n, :3], flat, topos[s])
+        # sums of up to n torques of size |x| |g|, in FP64
+        assert np.abs(gth[k0:k1] - ref).max() <= 1e-13 * flat.n * 100.0 * 10.0
+        assert np.abs(b.coords(s) - _sequential(x, topos[s], flat, delta[k0:k1])).max() < 1e-9
