@@ -274,7 +274,7 @@ __device__ bool team_rebuild(const MoveCtx &C, const MCConfigDev &cfg, int s, co
     const int32_t *ec = C.t.excl_cols;
     for (int i = a0 + wid; i < a1; i += nw) {
         int nf, nh, nsf, nsh;
-        nl_row_atom<0>(i, lane, g, b.xyz, rcut2, ws.cell_of, ws.cstart, ws.cell_atoms, b.prm64, cfg.reach_pad, ep, ec,
+        nl_row_atom<0>(i, lane, g, b.xyz, rcut2, ws.cell_of, CellStarts{start}, ws.cell_atoms, b.prm64, cfg.reach_pad, ep, ec,
                        C.t.excl_win, nl, nf, nh, nsf, nsh);
         if (lane == 0) {
             ws.cnt[i] = nf;
@@ -315,7 +315,7 @@ __device__ bool team_rebuild(const MoveCtx &C, const MCConfigDev &cfg, int s, co
     if (!__ldcg(&ws.flag[s])) return false;
     for (int i = a0 + wid; i < a1; i += nw) {
         int nf, nh, nsf, nsh;
-        nl_row_atom<1>(i, lane, g, b.xyz, rcut2, ws.cell_of, ws.cstart, ws.cell_atoms, b.prm64, cfg.reach_pad, ep, ec,
+        nl_row_atom<1>(i, lane, g, b.xyz, rcut2, ws.cell_of, CellStarts{start}, ws.cell_atoms, b.prm64, cfg.reach_pad, ep, ec,
                        C.t.excl_win, nl, nf, nh, nsf, nsh);
     }
     T.sync();

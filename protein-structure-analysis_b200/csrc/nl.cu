@@ -9,42 +9,34 @@
 // j != i (used by Born radii and the move kernels, where the order is
 // irrelevant).  Each entry carries the 1-2/1-3/SS exclusion flag in bit 31.
 //
-// Pipeline (all stream-ordered, no host sync):
-//   grid   : one CTA per system — FP64 bounding box, cell-grid shape
-//   offsets: one CTA — per-system cell offsets, capacity check
-//   bin    : atom -> cell, cell histogram
-//   scan   : cell starts
-//   scatter: atoms into cells, then a per-cell rank sort (ascending index)
-//   cellpos: FP32 positions (relative to the grid origin) and R* in cell
-//            order, so the row scan streams its candidates coalesced
-//   rows   : warp per atom — one scan stages the row in shared memory,
-//            takes space from the system's cursors, writes the four rows
-//            ballot-compacted in scan order
-//   final  : per system — entry counts, overflow flag
+// Three launches, all stream-ordered, no host sync:
+//   cells : one cluster per system — FP64 bounding box, grid shape, cell
+//           counts, cell starts, atoms scattered into their cells
+//   order : thread per atom — its rank in its cell (ascending index), and the
+//           cell-ordered copy of positions that the row scan streams
+//   rows  : warp per one or two neighbouring atoms — one scan of the 27 cells
+//           marks the candidates, then each row is staged in shared memory,
+//           takes space in the system's regions and is written
 // Every stage honours an optional per-system mask, so systems can be
 // rebuilt independently (the MC driver rebuilds only chains that drifted).
-#include <cstdio>
+#include <cooperative_groups.h>
 
 #include "alma_common.cuh"
-#include "alma_scan.cuh"
 #include "nl_core.cuh"
 
 namespace alma {
 
+namespace cg = cooperative_groups;
+
 struct NLWork {
-    SysGrid *grid;        // [nsys]
+    SysGrid *grid;        // [nsys]; ncell = 0: the grid did not fit
     int32_t *cell_of;     // [natoms] local cell index
-    int32_t *cell_count;  // [max_cells]
-    int32_t *cell_fill;   // [max_cells]
-    int64_t *cell_start;  // [max_cells+1]
-    int32_t *cell_atoms;  // [natoms]
-    float4 *cell_pos;     // [natoms] per cell slot: FP32 position relative to the grid origin, R*
-    int32_t *sort_spill;  // [natoms] rank-sort space for oversized cells
-    int64_t *tile_sums;   // scan scratch
-    int64_t *total_cells; // [1]
-    int32_t *ok;          // [1] 1 when the grid fit
-    int32_t *sys_ok;      // [nsys] 1 when the system's rows fit its region
-    int64_t *cursor;      // [4*nsys] next free entry of each row kind in the system's region
+    int32_t *cell_end;    // [max_cells] counts, then fill positions, then ends
+    int32_t *scattered;   // [natoms] atoms by cell, any order within a cell
+    int32_t *cell_atoms;  // [natoms] atoms by cell, ascending within a cell
+    float4 *cell_pos;     // [natoms + 32] per slot: FP32 position from the box centre, its square
+    float4 *cell_atom;    // [natoms] per slot: the same position, R*
+    unsigned long long *total_cells;  // [1] cells handed out
 };
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -56,373 +48,507 @@ static size_t carve(NLWork *w, char *base, int32_t nsys, int32_t natoms, int64_t
         off += align256(bytes);
         return p;
     };
-    const int64_t big = (max_cells + 1 > (int64_t)natoms + 1) ? max_cells + 1 : (int64_t)natoms + 1;
-    const int64_t ntiles = scan_num_tiles(big) + 1;
     NLWork t;
     t.grid = (SysGrid *)take(sizeof(SysGrid) * (size_t)(nsys > 0 ? nsys : 1));
     t.cell_of = (int32_t *)take(sizeof(int32_t) * (size_t)natoms);
-    t.cell_count = (int32_t *)take(sizeof(int32_t) * (size_t)max_cells);
-    t.cell_fill = (int32_t *)take(sizeof(int32_t) * (size_t)max_cells);
-    t.cell_start = (int64_t *)take(sizeof(int64_t) * (size_t)(max_cells + 1));
+    t.cell_end = (int32_t *)take(sizeof(int32_t) * (size_t)max_cells);
+    t.scattered = (int32_t *)take(sizeof(int32_t) * (size_t)natoms);
     t.cell_atoms = (int32_t *)take(sizeof(int32_t) * (size_t)natoms);
-    t.cell_pos = (float4 *)take(sizeof(float4) * (size_t)natoms);
-    t.sort_spill = (int32_t *)take(sizeof(int32_t) * (size_t)natoms);
-    t.tile_sums = (int64_t *)take(sizeof(int64_t) * (size_t)ntiles);
-    t.total_cells = (int64_t *)take(sizeof(int64_t));
-    t.ok = (int32_t *)take(sizeof(int32_t));
-    t.sys_ok = (int32_t *)take(sizeof(int32_t) * (size_t)(nsys > 0 ? nsys : 1));
-    t.cursor = (int64_t *)take(sizeof(int64_t) * 4 * (size_t)(nsys > 0 ? nsys : 1));
+    t.cell_pos = (float4 *)take(sizeof(float4) * ((size_t)natoms + 32));  // the scan reads whole chunks of 32
+    t.cell_atom = (float4 *)take(sizeof(float4) * (size_t)natoms);
+    t.total_cells = (unsigned long long *)take(sizeof(unsigned long long));
     if (w) *w = t;
     return off;
 }
 
-// One CTA per system: bounding box and grid shape (physics_engine.cpp:299-316).
-// A system outside the mask gets a 1x1x1 grid that no atom uses.
-__global__ void nl_grid_kernel(const int32_t *__restrict__ atom_off, const uint8_t *__restrict__ mask,
-                               const double *__restrict__ xyz, double nl_rcut2, SysGrid *__restrict__ grid) {
-    __shared__ double red[6][32];
-    const int s = blockIdx.x;
-    const int a0 = atom_off[s], a1 = (mask && !mask[s]) ? atom_off[s] : atom_off[s + 1];
+// Box centre of a grid: the origin of the FP32 copy of its atoms.
+__device__ __forceinline__ double3 grid_centre(const SysGrid &g) {
+    return make_double3(g.xlo + 0.5 * g.nx * g.cs, g.ylo + 0.5 * g.ny * g.cs, g.zlo + 0.5 * g.nz * g.cs);
+}
+
+// One cluster of CL CTAs per system: box and grid (physics_engine.cpp
+// :299-316), then count, scan and scatter of its atoms.  The per-system work
+// is a few dependent passes over its atoms and cells, so it runs as one
+// launch with cluster barriers instead of eight launches and two memsets over
+// all cells (one 65k-atom system: 125 us in eight kernels, of which the
+// bounding box by one CTA took 91; 33 us here).  Minima, maxima, counts
+// and cell contents do not depend on CL.
+constexpr int CELLS_THREADS = 512;
+
+template <int CL>
+__global__ void __launch_bounds__(CELLS_THREADS)
+nl_cells_kernel(const int32_t *__restrict__ atom_off, const uint8_t *__restrict__ mask,
+                const double *__restrict__ xyz, double nl_rcut2, int64_t max_cells, SysGrid *__restrict__ grid,
+                unsigned long long *total_cells, int32_t *cell_of, int32_t *cell_end, int32_t *__restrict__ scattered,
+                int64_t *__restrict__ need, uint32_t *status) {
+    constexpr int NW = CELLS_THREADS / 32, ITEMS = 4;
+    __shared__ double red[6][NW], box[6];
+    __shared__ long long cells_at;  // rank 0: first cell of the system, -1 when the grid does not fit
+    __shared__ int slice_total, warp_tot[NW];
+    const int rank = CL > 1 ? (int)cg::this_cluster().block_rank() : 0;
+    const int s = blockIdx.x / CL;
+    if (mask && !mask[s]) return;  // the whole cluster
+    auto sync = [] {
+        if constexpr (CL > 1) cg::this_cluster().sync();
+        else __syncthreads();
+    };
+    auto peer = [](auto *p, int r) {
+        if constexpr (CL > 1) return cg::this_cluster().map_shared_rank(p, r);
+        else return p;
+    };
+    const int a0 = atom_off[s], a1 = atom_off[s + 1];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int tid = rank * CELLS_THREADS + (int)threadIdx.x, nthr = CL * CELLS_THREADS;
+    // bounding box
     double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
-    for (int i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
+    for (int i = a0 + tid; i < a1; i += nthr) {
         const double4 p = ld_xyz(xyz, i);
         mn[0] = fmin(mn[0], p.x); mx[0] = fmax(mx[0], p.x);
         mn[1] = fmin(mn[1], p.y); mx[1] = fmax(mx[1], p.y);
         mn[2] = fmin(mn[2], p.z); mx[2] = fmax(mx[2], p.z);
     }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int d = 0; d < 3; ++d) {
-        double a = mn[d], b = mx[d];
         for (int o = 16; o > 0; o >>= 1) {
-            a = fmin(a, __shfl_xor_sync(0xffffffffu, a, o));
-            b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
+            mn[d] = fmin(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
+            mx[d] = fmax(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
         }
-        if (lane == 0) { red[d][wid] = a; red[3 + d][wid] = b; }
+        if (lane == 0) { red[d][wid] = mn[d]; red[3 + d][wid] = mx[d]; }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const int nw = blockDim.x >> 5;
-        double lo[3], hi[3];
-        for (int d = 0; d < 3; ++d) {
-            lo[d] = red[d][0]; hi[d] = red[3 + d][0];
-            for (int w = 1; w < nw; ++w) { lo[d] = fmin(lo[d], red[d][w]); hi[d] = fmax(hi[d], red[3 + d][w]); }
+    if (threadIdx.x < 6) {
+        double v = red[threadIdx.x][0];
+        for (int w = 1; w < NW; ++w)
+            v = threadIdx.x < 3 ? fmin(v, red[threadIdx.x][w]) : fmax(v, red[threadIdx.x][w]);
+        box[threadIdx.x] = v;
+    }
+    sync();
+    double lo[3], hi[3];
+    for (int d = 0; d < 3; ++d) {
+        lo[d] = *peer(&box[d], 0);
+        hi[d] = *peer(&box[3 + d], 0);
+        for (int r = 1; r < CL; ++r) {
+            lo[d] = fmin(lo[d], *peer(&box[d], r));
+            hi[d] = fmax(hi[d], *peer(&box[3 + d], r));
         }
-        SysGrid g = grid_from_box(lo, hi, nl_rcut2, a1 - a0);
+    }
+    SysGrid g = grid_from_box(lo, hi, nl_rcut2, a1 - a0);
+    if (rank == 0 && threadIdx.x == 0) {
+        // (the product in FP64 first: a box that far out of range does not fit in any case)
+        long long at = -1;
+        if ((double)g.nx * g.ny * g.nz <= (double)max_cells) {
+            at = (long long)atomicAdd(total_cells, (unsigned long long)g.ncell);
+            if (at + g.ncell > max_cells) at = -1;
+        }
+        if (at < 0) set_status(status, ALMA_ST_CELL_OVERFLOW);
+        cells_at = at;
+        g.cell_off = at < 0 ? 0 : at;
+        g.ncell = at < 0 ? 0 : g.ncell;
         grid[s] = g;
+        for (int k = 0; k < 4; ++k) need[4 * (size_t)s + k] = 0;  // the row kernel counts here
     }
-}
-
-__global__ void nl_offsets_kernel(int nsys, SysGrid *__restrict__ grid, int64_t max_cells,
-                                  int64_t *__restrict__ total_cells, int32_t *__restrict__ ok,
-                                  uint32_t *__restrict__ status) {
-    if (threadIdx.x != 0) return;
-    int64_t acc = 0;
-    for (int s = 0; s < nsys; ++s) {
-        grid[s].cell_off = acc;
-        acc += grid[s].ncell;
-    }
-    *total_cells = acc;
-    const int fits = acc <= max_cells;
-    *ok = fits;
-    if (!fits) set_status(status, ALMA_ST_CELL_OVERFLOW);
-}
-
-__global__ void nl_bin_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms,
-                              const uint8_t *__restrict__ mask, const double *__restrict__ xyz,
-                              const SysGrid *__restrict__ grid, const int32_t *__restrict__ ok,
-                              int32_t *__restrict__ cell_of, int32_t *__restrict__ cell_count) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= natoms || !*ok) return;
-    const int s = sys_of_atom(atom_off, nsys, i);
-    if (mask && !mask[s]) return;
-    const SysGrid g = grid[s];
-    const int c = cell_of_point(g, ld_xyz(xyz, i));
-    cell_of[i] = c;
-    atomicAdd(&cell_count[g.cell_off + c], 1);
-}
-
-__global__ void nl_scatter_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms,
-                                  const uint8_t *__restrict__ mask, const SysGrid *__restrict__ grid,
-                                  const int32_t *__restrict__ ok, const int32_t *__restrict__ cell_of,
-                                  const int64_t *__restrict__ cell_start, int32_t *__restrict__ cell_fill,
-                                  int32_t *__restrict__ cell_atoms) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= natoms || !*ok) return;
-    const int s = sys_of_atom(atom_off, nsys, i);
-    if (mask && !mask[s]) return;
-    const int64_t c = grid[s].cell_off + cell_of[i];
-    const int slot = atomicAdd(&cell_fill[c], 1);
-    cell_atoms[cell_start[c] + slot] = i;
-}
-
-// Sorts every cell's atom list ascending (the reference pushes atoms in
-// index order).  Rank sort: each element's position is the number of
-// smaller elements (indices are distinct).
-constexpr int SORT_SMEM = 2048;
-__global__ void nl_cellsort_kernel(const int64_t *__restrict__ total_cells, const int32_t *__restrict__ ok,
-                                   const int64_t *__restrict__ cell_start, int32_t *__restrict__ cell_atoms,
-                                   int32_t *__restrict__ spill) {
-    __shared__ int32_t buf[SORT_SMEM];
-    if (!*ok) return;
-    const int64_t nc = *total_cells;
-    for (int64_t c = blockIdx.x; c < nc; c += gridDim.x) {
-        const int64_t b = cell_start[c];
-        const int m = (int)(cell_start[c + 1] - b);
-        if (m <= 1) continue;
-        int32_t *src = cell_atoms + b;
-        if (m <= SORT_SMEM) {
-            for (int k = threadIdx.x; k < m; k += blockDim.x) buf[k] = src[k];
-            __syncthreads();
-            for (int k = threadIdx.x; k < m; k += blockDim.x) {
-                const int32_t v = buf[k];
-                int rank = 0;
-                for (int q = 0; q < m; ++q) rank += buf[q] < v;
-                src[rank] = v;
-            }
-            __syncthreads();
-        } else {
-            // Oversized cell: rank in global memory through the spill buffer
-            // (same positions as cell_atoms), then copy back.
-            int32_t *tmp = spill + b;
-            for (int k = threadIdx.x; k < m; k += blockDim.x) {
-                const int32_t v = src[k];
-                int rank = 0;
-                for (int q = 0; q < m; ++q) rank += src[q] < v;
-                tmp[rank] = v;
-            }
-            __syncthreads();
-            for (int k = threadIdx.x; k < m; k += blockDim.x) src[k] = tmp[k];
-            __syncthreads();
-        }
-    }
-}
-
-// Cell-ordered copy of the candidates' positions for the row scan: slot k
-// of cell_atoms gets its atom's position relative to its system's grid
-// origin in FP32 and its R* (the SASA-reach radius).  The 27-cell scan then
-// reads each 32-candidate chunk as one coalesced 512-byte load instead of
-// 32 scattered FP64 gathers; FP64 decides only inside the margin.
-__global__ void nl_cellpos_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms,
-                                  const int64_t *__restrict__ total_cells, const int32_t *__restrict__ ok,
-                                  const int64_t *__restrict__ cell_start, const int32_t *__restrict__ cell_atoms,
-                                  const SysGrid *__restrict__ grid, const double *__restrict__ xyz,
-                                  const double *__restrict__ prm64, float4 *__restrict__ cell_pos) {
-    if (!*ok) return;
-    const int64_t used = cell_start[*total_cells];
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < used && k < natoms;
-         k += (int64_t)gridDim.x * blockDim.x) {
-        const int j = cell_atoms[k];
-        const SysGrid g = grid[sys_of_atom(atom_off, nsys, j)];
-        const double4 p = ld_xyz(xyz, j);
-        cell_pos[k] = make_float4((float)(p.x - g.xlo), (float)(p.y - g.ylo), (float)(p.z - g.zlo),
-                                  prm64 ? (float)prm64[4 * (size_t)j + 1] : 0.0f);
-    }
-}
-
-// Entries of one row staged per warp in shared memory by the one-pass
-// build (48 KB per 8-warp block); a longer row is scanned a second time.
-constexpr int NL_STAGE = 1536;
-constexpr uint32_t NL_SHORT_BIT = 0x40000000u;  // staging only: the pair is within SASA reach
-
-// One-pass build, warp per atom: the 27-cell scan stages the row (exclusion
-// flag in bit 31, SASA-reach flag in bit 30) in shared memory in scan
-// order, lane 0 then takes space for the four rows from the system's
-// cursors (one atomic per row kind), and the warp writes the full row, the
-// half row (j > i) and the short rows from the staged entries — the same
-// rows, in the same order, as counting and filling in two scans.  Rows sit
-// in their system's region in the order the warps reach the cursors; every
-// reader goes through ptr/len.  A row that would overflow its region is not
-// written (nl_finalize_kernel raises the overflow); a row longer than the
-// stage is written by a second scan straight into its space.
-__global__ void __launch_bounds__(256, 4)
-nl_rows_onepass_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const uint8_t *__restrict__ mask,
-                       const double *__restrict__ xyz, double rcut2, const SysGrid *__restrict__ grid,
-                       const int32_t *__restrict__ ok, const int32_t *__restrict__ cell_of,
-                       const int64_t *__restrict__ cell_start, const int32_t *__restrict__ cell_atoms,
-                       const float4 *__restrict__ cell_pos, const double *__restrict__ prm64, double reach_pad,
-                       const int64_t *__restrict__ excl_ptr, const int32_t *__restrict__ excl_cols,
-                       const uint32_t *__restrict__ excl_win, AlmaNL nl, int64_t *__restrict__ cursor) {
-    extern __shared__ uint32_t nl_stage_smem[];
-    const int warps_per_block = blockDim.x >> 5;
-    const int i = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (i >= natoms || !*ok) return;
-    const int s = sys_of_atom(atom_off, nsys, i);
-    if (mask && !mask[s]) return;
-    const SysGrid g = grid[s];
-    uint32_t *stage = nl_stage_smem + (threadIdx.x >> 5) * NL_STAGE;
-    const bool shorts = nl.sfull_cols != nullptr;
-    const int c = cell_of[i];
-    const int cx = c % g.nx, cy = (c / g.nx) % g.ny, cz = c / (g.nx * g.ny);
-    const double4 pi = ld_xyz(xyz, i);
-    const double ri_pad = shorts ? prm64[4 * (size_t)i + 1] + reach_pad : 0.0;
-    const uint4 ew = excl_window_of(excl_win, i);
-    // the FP32 frame of the cell copy; r² within margin2 of a cutoff is
-    // decided in FP64, so the rows are those of the FP64 test bit for bit
-    const float pfx = (float)(pi.x - g.xlo), pfy = (float)(pi.y - g.ylo), pfz = (float)(pi.z - g.zlo);
-    const float m2 = g.margin2, cut_lo = (float)rcut2 - m2, cut_hi = (float)rcut2 + m2;
-    const float rpad_f = (float)ri_pad;
-    int nfull = 0, nhalf = 0, nsfull = 0, nshalf = 0;
-    int jmin = 0x7fffffff, jmax = -1;
-    const unsigned lt = (1u << lane) - 1u;
-    for (int dz = -1; dz <= 1; ++dz) {
-        const int cz2 = cz + dz;
-        if (cz2 < 0 || cz2 >= g.nz) continue;
-        for (int dy = -1; dy <= 1; ++dy) {
-            const int cy2 = cy + dy;
-            if (cy2 < 0 || cy2 >= g.ny) continue;
-            for (int dx = -1; dx <= 1; ++dx) {
-                const int cx2 = cx + dx;
-                if (cx2 < 0 || cx2 >= g.nx) continue;
-                const int64_t cell = g.cell_off + cx2 + (int64_t)g.nx * (cy2 + (int64_t)g.ny * cz2);
-                const int64_t beg = cell_start[cell], end = cell_start[cell + 1];
-                for (int64_t k0 = beg; k0 < end; k0 += 32) {
-                    const int64_t k = k0 + lane;
-                    int j = -1;
-                    bool in = false, sh = false;
-                    if (k < end) {
-                        j = cell_atoms[k];
-                        const float4 q = cell_pos[k];
-                        const float dx = q.x - pfx, dy = q.y - pfy, dz = q.z - pfz;
-                        const float r2f = dx * dx + dy * dy + dz * dz;
-                        if (r2f < cut_hi && j != i) {
-                            double r2 = -1.0;  // FP64 r², computed only when a test needs it
-                            if (r2f > cut_lo) {
-                                r2 = d2_of(pi, ld_xyz(xyz, j));
-                                in = r2 < rcut2;
-                            } else {
-                                in = true;
-                            }
-                            if (in && shorts) {
-                                const float rf = rpad_f + q.w, rf2 = rf * rf;
-                                if (r2f < rf2 - m2) {
-                                    sh = true;
-                                } else if (r2f <= rf2 + m2) {
-                                    if (r2 < 0.0) r2 = d2_of(pi, ld_xyz(xyz, j));
-                                    const double reach = ri_pad + prm64[4 * (size_t)j + 1];
-                                    sh = r2 < reach * reach;
-                                }
-                            }
-                        }
-                    }
-                    const unsigned mf = __ballot_sync(0xffffffffu, in);
-                    const int at = nfull + __popc(mf & lt);
-                    if (in) {
-                        jmin = min(jmin, j);
-                        jmax = max(jmax, j);
-                        if (at < NL_STAGE)
-                            stage[at] = (uint32_t)j |
-                                        (excluded_w(excl_win, ew, excl_ptr, excl_cols, i, j) ? ALMA_EXCL_BIT : 0u) |
-                                        (sh ? NL_SHORT_BIT : 0u);
-                    }
-                    // the other row kinds are counted from the stage after the
-                    // scan; only entries past its end (a rare long row) here
-                    if (nfull + __popc(mf) > NL_STAGE) {
-                        const bool over = in && at >= NL_STAGE;
-                        nhalf += __popc(__ballot_sync(0xffffffffu, over && j > i));
-                        nsfull += __popc(__ballot_sync(0xffffffffu, over && sh));
-                        nshalf += __popc(__ballot_sync(0xffffffffu, over && sh && j > i));
-                    }
-                    nfull += __popc(mf);
-                }
-            }
-        }
-    }
-    __syncwarp();
-    for (int t0 = 0; t0 < min(nfull, NL_STAGE); t0 += 32) {  // half / short counts of the staged entries
-        const int t = t0 + lane;
-        const uint32_t st = t < min(nfull, NL_STAGE) ? stage[t] : 0u;
-        const bool v = t < min(nfull, NL_STAGE);
-        const bool hf = v && (int)(st & ALMA_IDX_MASK & ~NL_SHORT_BIT) > i, sh = v && (st & NL_SHORT_BIT);
-        nhalf += __popc(__ballot_sync(0xffffffffu, hf));
-        nsfull += __popc(__ballot_sync(0xffffffffu, sh));
-        nshalf += __popc(__ballot_sync(0xffffffffu, hf && sh));
-    }
-    // space in the system's regions (relative offsets; -1: does not fit)
-    int64_t off[4] = {0, 0, 0, 0};
-    const int nkind = shorts ? 4 : 2;
-    if (lane == 0) {
-        const int n[4] = {nfull, nhalf, nsfull, nshalf};
-        const int64_t *basev[4] = {nl.full_base, nl.half_base, nl.sfull_base, nl.shalf_base};
-        for (int kd = 0; kd < nkind; ++kd) {
-            const int64_t o = atomicAdd(reinterpret_cast<unsigned long long *>(cursor + 4 * s + kd),
-                                        (unsigned long long)n[kd]);
-            off[kd] = o + n[kd] <= basev[kd][s + 1] - basev[kd][s] ? basev[kd][s] + o : -1;
-        }
-    }
-    for (int kd = 0; kd < 4; ++kd) off[kd] = __shfl_sync(0xffffffffu, off[kd], 0);
-    bool fits = true;
-    for (int kd = 0; kd < nkind; ++kd) fits = fits && off[kd] >= 0;
-    if (!fits) return;  // the system overflows: nl_finalize_kernel flags it
-    if (lane == 0) {
-        nl.full_ptr[i] = off[0];
-        nl.full_len[i] = nfull;
-        nl.half_ptr[i] = off[1];
-        nl.half_len[i] = nhalf;
-        if (shorts) {
-            nl.sfull_ptr[i] = off[2];
-            nl.sfull_len[i] = nsfull;
-            nl.shalf_ptr[i] = off[3];
-            nl.shalf_len[i] = nshalf;
-        }
-    }
-    if (nfull > NL_STAGE) {  // too long to stage: scan again, writing at the pointers just set
-        __syncwarp();
-        int a, bb, cc, dd;
-        nl_row_atom<1>(i, lane, g, xyz, rcut2, cell_of, cell_start, cell_atoms, prm64, reach_pad, excl_ptr, excl_cols,
-                       excl_win, nl, a, bb, cc, dd);
+    sync();
+    const long long at = *peer(&cells_at, 0);
+    if (at < 0) {
+        sync();  // rank 0 stays until every CTA has read its word
         return;
     }
-    __syncwarp();
-    if (lane == 0) *reinterpret_cast<double4 *>(nl.ref_xyz + 4 * (size_t)i) = pi;
-    int wf = 0, wh = 0, wsf = 0, wsh = 0;
-    for (int t0 = 0; t0 < nfull; t0 += 32) {
-        const int t = t0 + lane;
-        const bool v = t < nfull;
-        const uint32_t st = v ? stage[t] : 0u;
-        const uint32_t e = st & ~NL_SHORT_BIT;
-        const int j = (int)(st & ALMA_IDX_MASK & ~NL_SHORT_BIT);
-        const bool hf = v && j > i, sh = v && (st & NL_SHORT_BIT);
-        const unsigned mh = __ballot_sync(0xffffffffu, hf);
-        const unsigned msf = __ballot_sync(0xffffffffu, sh);
-        const unsigned msh = __ballot_sync(0xffffffffu, sh && hf);
-        if (v) nl.full_cols[off[0] + t] = e;
-        if (hf) nl.half_cols[off[1] + wh + __popc(mh & lt)] = e;
-        if (sh) {
-            nl.sfull_cols[off[2] + wsf + __popc(msf & lt)] = e;
-            if (hf) nl.shalf_cols[off[3] + wsh + __popc(msh & lt)] = e;
-        }
-        wf += 32;
-        wh += __popc(mh);
-        wsf += __popc(msf);
-        wsh += __popc(msh);
+    const int ncell = (int)g.ncell;  // <= max_cells, and a cell index is 32-bit
+    int32_t *end = cell_end + at;
+    for (int c = tid; c < ncell; c += nthr) end[c] = 0;
+    sync();
+    for (int i = a0 + tid; i < a1; i += nthr) {
+        const int c = cell_of_point(g, ld_xyz(xyz, i));
+        cell_of[i] = c;
+        atomicAdd(&end[c], 1);
     }
-    (void)wf;
-    if (nl.full_span != nullptr) {
-        jmin = __reduce_min_sync(0xffffffffu, jmin);
-        jmax = __reduce_max_sync(0xffffffffu, jmax);
-        if (lane == 0) {
-            nl.full_span[2 * (size_t)i] = jmin;
-            nl.full_span[2 * (size_t)i + 1] = jmax;
+    sync();
+    // counts -> first slots: each CTA scans a slice of the cells behind the
+    // totals of the slices before it
+    const int per = (ncell + CL - 1) / CL, c0 = min(ncell, rank * per), c1 = min(ncell, c0 + per);
+    if constexpr (CL > 1) {
+        int sum = 0;
+        for (int c = c0 + (int)threadIdx.x; c < c1; c += CELLS_THREADS) sum += end[c];
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0) warp_tot[wid] = sum;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int t = 0;
+            for (int w = 0; w < NW; ++w) t += warp_tot[w];
+            slice_total = t;
         }
+        sync();
+    }
+    int carry = a0;
+    for (int r = 0; r < rank; ++r) carry += *peer(&slice_total, r);
+    for (int b0 = c0; b0 < c1; b0 += CELLS_THREADS * ITEMS) {
+        int v[ITEMS], sum = 0;
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const int c = b0 + (int)threadIdx.x * ITEMS + k;
+            v[k] = c < c1 ? end[c] : 0;
+            sum += v[k];
+        }
+        int inc = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        __syncthreads();  // the warp totals of the last chunk have been read
+        if (lane == 31) warp_tot[wid] = inc;
+        __syncthreads();
+        int at_ = carry + inc - sum;
+        for (int w = 0; w < NW; ++w) {
+            const int t = warp_tot[w];
+            if (w < wid) at_ += t;
+            carry += t;
+        }
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const int c = b0 + (int)threadIdx.x * ITEMS + k;
+            if (c < c1) end[c] = at_;
+            at_ += v[k];
+        }
+    }
+    sync();
+    for (int i = a0 + tid; i < a1; i += nthr) scattered[atomicAdd(&end[cell_of[i]], 1)] = i;
+    // (every slot advanced by its cell's count: end[] now holds the cell ends)
+}
+
+// Thread per atom: its place in its cell is the number of smaller indices
+// there (the reference pushes atoms in index order).  The threads of a warp
+// mostly share a cell, so the reads are broadcasts.
+__global__ void __launch_bounds__(256)
+nl_order_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const uint8_t *__restrict__ mask,
+                const SysGrid *__restrict__ grid, const int32_t *__restrict__ cell_of,
+                const int32_t *__restrict__ cell_end, const int32_t *__restrict__ scattered,
+                const double *__restrict__ xyz, const double *__restrict__ prm64, int32_t *__restrict__ cell_atoms,
+                float4 *__restrict__ cell_pos, float4 *__restrict__ cell_atom) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= natoms) return;
+    const int s = sys_of_atom(atom_off, nsys, i);
+    if (mask && !mask[s]) return;
+    const SysGrid g = grid[s];
+    if (g.ncell == 0) return;
+    const CellEnds cells{cell_end + g.cell_off, atom_off[s]};
+    int64_t beg, end;
+    cells(cell_of[i], beg, end);
+    int at = (int)beg;
+#pragma unroll 8
+    for (int q = (int)beg; q < (int)end; ++q) at += scattered[q] < i;
+    const double4 p = ld_xyz(xyz, i);
+    const double3 o = grid_centre(g);
+    const float x = (float)(p.x - o.x), y = (float)(p.y - o.y), z = (float)(p.z - o.z);
+    cell_atoms[at] = i;
+    cell_pos[at] = make_float4(x, y, z, x * x + y * y + z * z);
+    cell_atom[at] = make_float4(x, y, z, prm64 ? (float)prm64[4 * (size_t)i + 1] : 0.0f);
+}
+
+// Row scan.  The candidates of an atom are the atoms of 27 cells: nine runs
+// of three x-neighbours, each contiguous in the cell-ordered copy and already
+// in the reference's scan order.  A warp takes G consecutive slots (atoms of
+// one cell, or of neighbouring cells of one run: the run is then wider, which
+// only adds candidates) and streams the runs once for all of them:
+//   scan   |q|² - 2 p.q < 14² - |p|² in three FP32 FMAs per candidate, with a
+//          margin that covers their rounding; the ballot of a chunk goes to
+//          shared memory, chunks without a candidate are dropped
+//   stage  the bits of each atom's masks become a list of slots
+//   decide per staged slot, all lanes busy: the FP32 distance (coordinates
+//          relative to the box centre), FP64 within fp32_margin2 of a cutoff,
+//          the exclusion bit, the SASA reach — the rows are those of the FP64
+//          tests bit for bit
+//   write  space from the system's counters (one atomic per row kind, which
+//          are also the entry counts), then the four rows, ballot-compacted
+// Issue and L1 latency bound it (24-28 warps per SM by registers and shared
+// memory).  The scan before this one compacted every chunk of 27 separate
+// cells as it went, about 12,000 issue slots per atom at 600 neighbours.  65k
+// atoms: 1,010 -> 445 us; 48 x 4.8k atoms: 1,892 -> 978 us.  Rows sit in their system's region in any order; a row that
+// would overflow it is not written and raises the flag.
+constexpr int NL_STAGE = 1280;  // staged entries of a row; a longer one is scanned in FP64
+constexpr int NL_CHUNKS = 160;  // chunks of 32 candidates that hold one within reach; likewise
+constexpr int NL_WARPS = 4;
+constexpr uint32_t NL_SHORT_BIT = 0x40000000u;  // staging only: the pair is within SASA reach
+constexpr uint32_t NL_DROPPED = 0xffffffffu;    // staging only: not an entry (2^30 - 2 is the largest index)
+
+template <int G>
+struct RowSmem {
+    uint32_t stage[NL_STAGE];
+    uint32_t bits[G][NL_CHUNKS];
+    int32_t base[NL_CHUNKS];
+};
+
+// Space for the rows of atom i (n: entries per row kind in lanes 0-3): the
+// offset of kind k in lane k, or false when a region is full.
+__device__ __forceinline__ bool take_rows(const AlmaNL &nl, int s, int n, int lane, int nkind, int64_t &off,
+                                          uint32_t *status) {
+    bool fits = true;
+    if (lane < nkind) {
+        const int64_t *b = lane == 0 ? nl.full_base : lane == 1 ? nl.half_base : lane == 2 ? nl.sfull_base
+                                                                                           : nl.shalf_base;
+        const int64_t o = (int64_t)atomicAdd(reinterpret_cast<unsigned long long *>(nl.need + 4 * (size_t)s + lane),
+                                             (unsigned long long)n);
+        const int64_t beg = b[s];
+        off = beg + o;
+        fits = off + n <= b[s + 1];
+    }
+    if (__all_sync(0xffffffffu, fits)) return true;
+    if (lane == 0) set_status(status, ALMA_ST_NL_OVERFLOW);
+    return false;
+}
+
+__device__ __forceinline__ void set_rows(const AlmaNL &nl, int i, int n, int lane, int nkind, int64_t off) {
+    if (lane < nkind) {
+        (lane == 0 ? nl.full_ptr : lane == 1 ? nl.half_ptr : lane == 2 ? nl.sfull_ptr : nl.shalf_ptr)[i] = off;
+        (lane == 0 ? nl.full_len : lane == 1 ? nl.half_len : lane == 2 ? nl.sfull_len : nl.shalf_len)[i] = n;
     }
 }
 
-// Per system after the one-pass build: entry counts into need[], overflow
-// into the status word.
-__global__ void nl_finalize_kernel(int nsys, const uint8_t *__restrict__ mask, const int32_t *__restrict__ ok,
-                                   const int64_t *__restrict__ cursor, AlmaNL nl, uint32_t *__restrict__ status) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nsys || !*ok || (mask && !mask[s])) return;
-    const int nkind = nl.sfull_cols ? 4 : 2;
-    const int64_t *basev[4] = {nl.full_base, nl.half_base, nl.sfull_base, nl.shalf_base};
-    bool fits = true;
-    for (int kd = 0; kd < nkind; ++kd) {
-        const int64_t n = cursor[4 * s + kd];
-        nl.need[4 * s + kd] = n;
-        fits = fits && n <= basev[kd][s + 1] - basev[kd][s];
+template <int G>
+__global__ void __launch_bounds__(NL_WARPS * 32, G == 1 ? 8 : 7)
+nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const uint8_t *__restrict__ mask,
+               const double *__restrict__ xyz, double rcut2, const SysGrid *__restrict__ grid,
+               const int32_t *__restrict__ cell_of, const int32_t *__restrict__ cell_end,
+               const int32_t *__restrict__ cell_atoms, const float4 *__restrict__ cell_pos,
+               const float4 *__restrict__ cell_atom, const double *__restrict__ prm64, double reach_pad,
+               const int64_t *__restrict__ excl_ptr, const int32_t *__restrict__ excl_cols,
+               const uint32_t *__restrict__ excl_win, AlmaNL nl, uint32_t *status) {
+    __shared__ RowSmem<G> smem[NL_WARPS];
+    RowSmem<G> &W = smem[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int p0 = (blockIdx.x * NL_WARPS + (threadIdx.x >> 5)) * G;
+    if (p0 >= natoms) return;
+    const bool shorts = nl.sfull_cols != nullptr;
+    const int nkind = shorts ? 4 : 2;
+    // lane g < G: the atom of slot p0 + g and its cell
+    int my_s = -1, my_i = 0, my_cx = 0, my_row = -1;
+    if (lane < G && p0 + lane < natoms) {
+        const int s = sys_of_atom(atom_off, nsys, p0 + lane);
+        if ((!mask || mask[s]) && grid[s].ncell > 0) {
+            my_s = s;
+            my_i = cell_atoms[p0 + lane];
+            const int c = cell_of[my_i], nx = grid[s].nx;
+            my_cx = c % nx;
+            my_row = c / nx;
+        }
     }
-    if (!fits) set_status(status, ALMA_ST_NL_OVERFLOW);
+    unsigned todo = __ballot_sync(0xffffffffu, my_s >= 0);
+    while (todo) {
+        const int lead = __ffs(todo) - 1;
+        const int s = __shfl_sync(0xffffffffu, my_s, lead), row = __shfl_sync(0xffffffffu, my_row, lead);
+        const bool mine = my_s == s && my_row == row;
+        const unsigned mem = __ballot_sync(0xffffffffu, mine) & todo;
+        todo &= ~mem;
+        const SysGrid g = grid[s];
+        const CellEnds cells{cell_end + g.cell_off, atom_off[s]};
+        const int x0 = max(0, __reduce_min_sync(0xffffffffu, mine ? my_cx : 0x7fffffff) - 1);
+        const int x1 = min(g.nx - 1, __reduce_max_sync(0xffffffffu, mine ? my_cx : -1) + 1);
+        // lane r < 9: run r in (dz, dy) order
+        int rbeg = 0, rend = 0;
+        if (lane < 9) {
+            const int y = row % g.ny + lane % 3 - 1, z = row / g.ny + lane / 3 - 1;
+            if (y >= 0 && y < g.ny && z >= 0 && z < g.nz) {
+                const int64_t c = (int64_t)g.nx * (y + (int64_t)g.ny * z);
+                rbeg = cells.beg(c + x0);
+                rend = cells.end_[c + x1];
+            }
+        }
+        // |p|² and the products round to within 2^-24 of terms up to 3/4
+        // E² (E the longest side): 16 roundings of that size, twice over
+        const float ext = (float)(fmax(g.nx, fmax(g.ny, g.nz)) * g.cs);
+        const float m2 = g.margin2, cut_lo = (float)rcut2 - m2, cut_hi = (float)rcut2 + m2;
+        const float cut_scan = cut_hi + 32.0f * 0.75f * 5.9604645e-8f * ext * ext;
+        float ax[G], ay[G], az[G], thr[G];
+#pragma unroll
+        for (int a = 0; a < G; ++a) {
+            const float4 q = cell_pos[p0 + ((mem >> a) & 1u ? a : lead)];
+            ax[a] = -2.0f * q.x;
+            ay[a] = -2.0f * q.y;
+            az[a] = -2.0f * q.z;
+            thr[a] = cut_scan - q.w;
+        }
+        // the runs as one list of chunks: lane r < 9 holds its run's chunks
+        const int nck = (rend - rbeg + 31) >> 5;
+        int upto = nck;  // chunks of the runs up to and with this one
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += u;
+        }
+        const int total = __shfl_sync(0xffffffffu, upto, 8);
+        const unsigned lt = (1u << lane) - 1u;
+        int nch = 0;
+        for (int c0 = 0; c0 < total; c0 += 32) {
+            // this lane's chunk: where it starts and which of its lanes exist
+            int from = 0, left = 0;
+#pragma unroll
+            for (int r = 0; r < 9; ++r) {
+                const int e = __shfl_sync(0xffffffffu, upto, r), n = __shfl_sync(0xffffffffu, nck, r);
+                const int beg = __shfl_sync(0xffffffffu, rbeg, r), end = __shfl_sync(0xffffffffu, rend, r);
+                const int at = c0 + lane - (e - n);
+                if (at >= 0 && at < n) {
+                    from = beg + 32 * at;
+                    left = end - from;
+                }
+            }
+            uint32_t keep[G];
+#pragma unroll
+            for (int a = 0; a < G; ++a) keep[a] = 0u;
+            const int nin = min(32, total - c0);
+            for (int c = 0; c < nin; c += 4) {  // four independent loads in flight
+                float4 q[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) q[u] = cell_pos[__shfl_sync(0xffffffffu, from, c + u) + lane];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int a = 0; a < G; ++a) {
+                        const float t = fmaf(ax[a], q[u].x, fmaf(ay[a], q[u].y, fmaf(az[a], q[u].z, q[u].w)));
+                        const uint32_t m = __ballot_sync(0xffffffffu, t < thr[a]);
+                        keep[a] = lane == c + u ? m : keep[a];
+                    }
+            }
+            // chunks with a candidate, compacted
+            const uint32_t exist = left >= 32 ? 0xffffffffu : left > 0 ? (1u << left) - 1u : 0u;
+            uint32_t any = 0u;
+#pragma unroll
+            for (int a = 0; a < G; ++a) any |= keep[a] &= exist;
+            const unsigned some = __ballot_sync(0xffffffffu, any != 0u);
+            const int at = nch + __popc(some & lt);
+            if (any != 0u && at < NL_CHUNKS) {
+                W.base[at] = from;
+#pragma unroll
+                for (int a = 0; a < G; ++a) W.bits[a][at] = keep[a];
+            }
+            nch += __popc(some);
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int a = 0; a < G; ++a) {
+            if (!((mem >> a) & 1u)) continue;
+            const int i = __shfl_sync(0xffffffffu, my_i, a);
+            const double4 pi = ld_xyz(xyz, i);
+            const double ri_pad = shorts ? prm64[4 * (size_t)i + 1] + reach_pad : 0.0;
+            int n = nch <= NL_CHUNKS ? 0 : NL_STAGE + 1;
+            for (int b = 0; b < nch && n <= NL_STAGE; b += 32) {
+                uint32_t m = b + lane < nch ? W.bits[a][b + lane] : 0u;
+                const int32_t from = b + lane < nch ? W.base[b + lane] : 0;
+                const int cnt = __popc(m);
+                int inc = cnt;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= o) inc += u;
+                }
+                int at = n + inc - cnt;
+                n += __shfl_sync(0xffffffffu, inc, 31);
+                if (n <= NL_STAGE)
+                    while (m) {
+                        W.stage[at++] = (uint32_t)(from + __ffs(m) - 1);
+                        m &= m - 1u;
+                    }
+            }
+            int64_t off = 0;
+            if (n > NL_STAGE) {  // too long to stage: counted, then written, by FP64 scans
+                int c[4];
+                nl_row_atom<0>(i, lane, g, xyz, rcut2, cell_of, cells, cell_atoms, prm64, reach_pad, excl_ptr,
+                               excl_cols, excl_win, nl, c[0], c[1], c[2], c[3]);
+                const int cnt = lane == 0 ? c[0] : lane == 1 ? c[1] : lane == 2 ? c[2] : c[3];
+                if (take_rows(nl, s, cnt, lane, nkind, off, status)) {
+                    set_rows(nl, i, cnt, lane, nkind, off);
+                    __syncwarp();
+                    nl_row_atom<1>(i, lane, g, xyz, rcut2, cell_of, cells, cell_atoms, prm64, reach_pad, excl_ptr,
+                                   excl_cols, excl_win, nl, c[0], c[1], c[2], c[3]);
+                }
+                continue;
+            }
+            __syncwarp();
+            const float4 pf = cell_atom[p0 + a];
+            const float rpad_f = (float)ri_pad;
+            const uint4 ew = excl_window_of(excl_win, i);
+            int cf = 0, cs = 0;  // this lane's entries: full | half << 16, short full | short half << 16
+            int jmin = 0x7fffffff, jmax = -1;
+#pragma unroll 2
+            for (int t = lane; t < n; t += 32) {
+                const int k = (int)W.stage[t];
+                const int j = cell_atoms[k];
+                const float4 q = cell_atom[k];
+                const float dx = q.x - pf.x, dy = q.y - pf.y, dz = q.z - pf.z;
+                const float r2f = dx * dx + dy * dy + dz * dz;
+                uint32_t e = NL_DROPPED;
+                if (r2f < cut_hi && j != i) {
+                    double r2 = -1.0;  // FP64 r², computed only when a test needs it
+                    bool in = true, sh = false;
+                    if (r2f > cut_lo) {
+                        r2 = d2_of(pi, ld_xyz(xyz, j));
+                        in = r2 < rcut2;
+                    }
+                    if (in && shorts) {
+                        const float rf = rpad_f + q.w, rf2 = rf * rf;
+                        if (r2f < rf2 - m2) {
+                            sh = true;
+                        } else if (r2f <= rf2 + m2) {
+                            if (r2 < 0.0) r2 = d2_of(pi, ld_xyz(xyz, j));
+                            const double reach = ri_pad + prm64[4 * (size_t)j + 1];
+                            sh = r2 < reach * reach;
+                        }
+                    }
+                    if (in) {
+                        e = (uint32_t)j |
+                            (excluded_w(excl_win, ew, excl_ptr, excl_cols, i, j) ? ALMA_EXCL_BIT : 0u) |
+                            (sh ? NL_SHORT_BIT : 0u);
+                        const int up = j > i ? 0x10001 : 1;
+                        cf += up;
+                        cs += sh ? up : 0;
+                        jmin = min(jmin, j);
+                        jmax = max(jmax, j);
+                    }
+                }
+                W.stage[t] = e;
+            }
+            cf = __reduce_add_sync(0xffffffffu, cf);
+            cs = __reduce_add_sync(0xffffffffu, cs);
+            const int cnt = lane == 0 ? cf & 0xffff : lane == 1 ? cf >> 16 : lane == 2 ? cs & 0xffff : cs >> 16;
+            if (!take_rows(nl, s, cnt, lane, nkind, off, status)) {
+                __syncwarp();
+                continue;
+            }
+            set_rows(nl, i, cnt, lane, nkind, off);
+            if (lane == 0) *reinterpret_cast<double4 *>(nl.ref_xyz + 4 * (size_t)i) = pi;
+            if (nl.full_span != nullptr) {
+                jmin = __reduce_min_sync(0xffffffffu, jmin);
+                jmax = __reduce_max_sync(0xffffffffu, jmax);
+                if (lane == 0) {
+                    nl.full_span[2 * (size_t)i] = jmin;
+                    nl.full_span[2 * (size_t)i + 1] = jmax;
+                }
+            }
+            uint32_t *wf = nl.full_cols + __shfl_sync(0xffffffffu, off, 0);
+            uint32_t *wh = nl.half_cols + __shfl_sync(0xffffffffu, off, 1);
+            uint32_t *wsf = shorts ? nl.sfull_cols + __shfl_sync(0xffffffffu, off, 2) : nullptr;
+            uint32_t *wsh = shorts ? nl.shalf_cols + __shfl_sync(0xffffffffu, off, 3) : nullptr;
+            for (int t0 = 0; t0 < n; t0 += 32) {
+                const uint32_t st = t0 + lane < n ? W.stage[t0 + lane] : NL_DROPPED;
+                const bool v = st != NL_DROPPED;
+                const bool hf = v && (int)(st & (ALMA_IDX_MASK & ~NL_SHORT_BIT)) > i;
+                const unsigned mf = __ballot_sync(0xffffffffu, v), mh = __ballot_sync(0xffffffffu, hf);
+                const uint32_t e = st & ~NL_SHORT_BIT;
+                if (v) wf[__popc(mf & lt)] = e;
+                if (hf) wh[__popc(mh & lt)] = e;
+                wf += __popc(mf);
+                wh += __popc(mh);
+                if (shorts) {
+                    const bool sh = v && (st & NL_SHORT_BIT);
+                    const unsigned ms = __ballot_sync(0xffffffffu, sh), msh = ms & mh;
+                    if (sh) {
+                        wsf[__popc(ms & lt)] = e;
+                        if (hf) wsh[__popc(msh & lt)] = e;
+                    }
+                    wsf += __popc(ms);
+                    wsh += __popc(msh);
+                }
+            }
+            __syncwarp();  // the stage is the next atom's
+        }
+    }
 }
 
 // Exclusion windows (alma_excl_window): thread per atom over its CSR row
@@ -493,30 +619,36 @@ extern "C" int alma_nl_build(const AlmaBatch *b, const AlmaTopo *t, AlmaNL *nl, 
     NLWork w;
     carve(&w, (char *)workspace, nsys, natoms, max_cells);
     if (natoms == 0) return ALMA_OK;
-    ALMA_CUDA_TRY(cudaMemsetAsync(w.cell_count, 0, sizeof(int32_t) * (size_t)max_cells, st));
-    ALMA_CUDA_TRY(cudaMemsetAsync(w.cell_fill, 0, sizeof(int32_t) * (size_t)max_cells, st));
+    ALMA_CUDA_TRY(cudaMemsetAsync(w.total_cells, 0, sizeof(unsigned long long), st));
     const double rcut2 = (12.0 + 2.0) * (12.0 + 2.0);
-    nl_grid_kernel<<<nsys, 256, 0, st>>>(b->atom_off, sys_mask, b->xyz, rcut2, w.grid);
-    nl_offsets_kernel<<<1, 32, 0, st>>>(nsys, w.grid, max_cells, w.total_cells, w.ok, b->status);
-    const int tb = 256, nb = (natoms + tb - 1) / tb;
-    nl_bin_kernel<<<nb, tb, 0, st>>>(b->atom_off, nsys, natoms, sys_mask, b->xyz, w.grid, w.ok, w.cell_of,
-                                     w.cell_count);
-    exclusive_scan<int32_t>(w.cell_count, w.cell_start, max_cells, w.tile_sums, st);
-    nl_scatter_kernel<<<nb, tb, 0, st>>>(b->atom_off, nsys, natoms, sys_mask, w.grid, w.ok, w.cell_of, w.cell_start,
-                                         w.cell_fill, w.cell_atoms);
-    // oversized cells (> SORT_SMEM atoms) sort through the spill space
-    nl_cellsort_kernel<<<1184, 256, 0, st>>>(w.total_cells, w.ok, w.cell_start, w.cell_atoms, w.sort_spill);
-    nl_cellpos_kernel<<<nb, tb, 0, st>>>(b->atom_off, nsys, natoms, w.total_cells, w.ok, w.cell_start, w.cell_atoms,
-                                         w.grid, b->xyz, b->prm64, w.cell_pos);
-    const int wpb = 8, rb = (natoms + wpb - 1) / wpb;
+    // Four atoms per thread, up to 8 CTAs (the portable cluster): a cluster
+    // barrier costs as much as a few more atoms per thread (1,089 atoms: 7 us
+    // with one CTA, 10.5 with two; 200 x 4.9k atoms: 60 us, 119 at two atoms).
+    const int avg = natoms / nsys, unit = 4 * CELLS_THREADS;
+    const int cl = avg <= unit ? 1 : avg <= 2 * unit ? 2 : avg <= 4 * unit ? 4 : 8;
+    auto cells = cl == 1 ? nl_cells_kernel<1> : cl == 2 ? nl_cells_kernel<2> : cl == 4 ? nl_cells_kernel<4>
+                                                                                     : nl_cells_kernel<8>;
+    ALMA_CUDA_TRY(alma_launch_cluster(cells, (unsigned)nsys * (unsigned)cl, CELLS_THREADS, (unsigned)cl, (size_t)0,
+                                      st, b->atom_off, sys_mask, b->xyz, rcut2, max_cells, w.grid, w.total_cells,
+                                      w.cell_of, w.cell_end, w.scattered, nl->need, b->status));
+    nl_order_kernel<<<(natoms + 255) / 256, 256, 0, st>>>(b->atom_off, nsys, natoms, sys_mask, w.grid, w.cell_of,
+                                                          w.cell_end, w.scattered, b->xyz, b->prm64, w.cell_atoms,
+                                                          w.cell_pos, w.cell_atom);
     const int64_t *ep = t ? t->excl_ptr : nullptr;
     const int32_t *ec = t ? t->excl_cols : nullptr;
     const uint32_t *ew = t && t->excl_ptr ? t->excl_win : nullptr;
-    ALMA_CUDA_TRY(cudaMemsetAsync(w.cursor, 0, sizeof(int64_t) * 4 * (size_t)nsys, st));
-    nl_rows_onepass_kernel<<<rb, wpb * 32, sizeof(uint32_t) * NL_STAGE * wpb, st>>>(
-        b->atom_off, nsys, natoms, sys_mask, b->xyz, rcut2, w.grid, w.ok, w.cell_of, w.cell_start, w.cell_atoms,
-        w.cell_pos, b->prm64, reach_pad, ep, ec, ew, *nl, w.cursor);
-    nl_finalize_kernel<<<(nsys + 255) / 256, 256, 0, st>>>(nsys, sys_mask, w.ok, w.cursor, *nl, b->status);
-    ALMA_LAUNCH_CHECK_N("alma_nl_build", 11);
+    // Two atoms per warp read each candidate once for both; below about two
+    // waves of one-atom warps the chip has room for the shorter chains (16k
+    // atoms: 95 us with one, 98 with two; 32k: 203 and 194; 65k: 481 and 445;
+    // four per warp: 125, 222 and 474).
+    auto rows = [&](auto kfn, int per_warp) {
+        const int per_block = per_warp * NL_WARPS;
+        kfn<<<(natoms + per_block - 1) / per_block, NL_WARPS * 32, 0, st>>>(
+            b->atom_off, nsys, natoms, sys_mask, b->xyz, rcut2, w.grid, w.cell_of, w.cell_end, w.cell_atoms,
+            w.cell_pos, w.cell_atom, b->prm64, reach_pad, ep, ec, ew, *nl, b->status);
+    };
+    if (natoms >= 24000) rows(nl_rows_kernel<2>, 2);
+    else rows(nl_rows_kernel<1>, 1);
+    ALMA_LAUNCH_CHECK_N("alma_nl_build", 3);
     return ALMA_OK;
 }

@@ -44,6 +44,27 @@ __device__ __forceinline__ SysGrid grid_from_box(const double lo[3], const doubl
     return g;
 }
 
+// Slots [beg, end) of cell c's atoms, from absolute starts with a sentinel.
+struct CellStarts {
+    const int64_t *start;  // of the system: [ncell + 1]
+    __device__ __forceinline__ void operator()(int64_t c, int64_t &beg, int64_t &end) const {
+        beg = start[c];
+        end = start[c + 1];
+    }
+};
+
+// The same from cell ends: a cell starts where the one before it ends, the
+// first at the system's first slot.
+struct CellEnds {
+    const int32_t *end_;  // of the system: [ncell]
+    int32_t first;
+    __device__ __forceinline__ int beg(int64_t c) const { return c > 0 ? end_[c - 1] : first; }
+    __device__ __forceinline__ void operator()(int64_t c, int64_t &b, int64_t &e) const {
+        b = beg(c);
+        e = end_[c];
+    }
+};
+
 __device__ __forceinline__ int cell_of_point(const SysGrid &g, double4 p) {
     const int cx = min(g.nx - 1, max(0, (int)floor((p.x - g.xlo) / g.cs)));
     const int cy = min(g.ny - 1, max(0, (int)floor((p.y - g.ylo) / g.cs)));
@@ -91,11 +112,11 @@ __device__ __forceinline__ bool excluded_w(const uint32_t *win, uint4 w, const i
 // The rows of atom i, one warp (27 cells in (dz, dy, dx) order, ascending
 // atoms per cell, ballot-compacted).  PASS 0 counts (full, half, short full,
 // short half); PASS 1 writes the rows at the list's pointers and ref_xyz.
-// cell_start[g.cell_off + c] are absolute positions in cell_atoms.
-template <int PASS>
+// cells(c, beg, end) gives the slots of the system's cell c in cell_atoms.
+template <int PASS, typename Cells>
 __device__ __forceinline__ void nl_row_atom(int i, int lane, const SysGrid &g, const double *__restrict__ xyz,
                                             double rcut2, const int32_t *__restrict__ cell_of,
-                                            const int64_t *__restrict__ cell_start,
+                                            const Cells &cells,
                                             const int32_t *__restrict__ cell_atoms, const double *__restrict__ prm64,
                                             double reach_pad, const int64_t *__restrict__ excl_ptr,
                                             const int32_t *__restrict__ excl_cols, const uint32_t *excl_win,
@@ -127,8 +148,8 @@ __device__ __forceinline__ void nl_row_atom(int i, int lane, const SysGrid &g, c
             for (int dx = -1; dx <= 1; ++dx) {
                 const int cx2 = cx + dx;
                 if (cx2 < 0 || cx2 >= g.nx) continue;
-                const int64_t cell = g.cell_off + cx2 + (int64_t)g.nx * (cy2 + (int64_t)g.ny * cz2);
-                const int64_t beg = cell_start[cell], end = cell_start[cell + 1];
+                int64_t beg, end;
+                cells(cx2 + (int64_t)g.nx * (cy2 + (int64_t)g.ny * cz2), beg, end);
                 for (int64_t k0 = beg; k0 < end; k0 += 32) {
                     const int64_t k = k0 + lane;
                     int j = -1;

@@ -304,11 +304,11 @@ class DeviceBatch:
             if st & (_lib.ST_NL_OVERFLOW | _lib.ST_CELL_OVERFLOW):
                 need = self.need.cpu().numpy()
                 self.status.zero_()
-                if st & _lib.ST_CELL_OVERFLOW:
+                if st & _lib.ST_CELL_OVERFLOW:  # a system whose grid did not fit has no row counts yet
                     self.max_cells *= 4
                     self.nl_ws = torch.zeros(self.L.alma_nl_workspace_bytes(self.nsys, self.natoms, self.max_cells),
                                              dtype=torch.uint8, device=_DEV)
-                if st & _lib.ST_NL_OVERFLOW:
+                else:
                     keep_cells = self.max_cells
                     self._alloc_nl(need)
                     self.max_cells = keep_cells

@@ -323,3 +323,41 @@ def test_exclusion_window(golden):
     for a, c in zip(with_win, csr):
         for x, y in zip(a, c):
             assert np.array_equal(x, y)
+
+
+def _clouds(kind):
+    rng = np.random.default_rng(11)
+    if kind == "tiny":  # around a chunk, and a chain of one atom
+        return [rng.uniform(0, 20, (n, 3)) for n in (1, 2, 31, 32, 33, 95)]
+    if kind == "long rows":  # more neighbours than a row's stage, more chunks than its mask list
+        return [rng.uniform(0, 11, (1400, 3)), rng.uniform(0, 60, (700, 3)), rng.uniform(0, 24, (5600, 3))]
+    if kind == "stretched":  # a long thin box far from the origin: wide FP32 margins, mostly empty cells
+        x = rng.uniform(0, 1, (3000, 3)) * [2500.0, 30.0, 20.0] + [4.0e4, -3.0e4, 10.0]
+        return [x, rng.uniform(0, 25, (40, 3))]
+    # two atoms per warp, uneven systems whose slots meet inside a warp
+    return [rng.uniform(0, 18 + 4 * k, (1501 + 1200 * k, 3)) for k in range(6)]
+
+
+@pytest.mark.parametrize("kind", ["tiny", "long rows", "stretched", "two per warp"])
+def test_nl_rows_at_the_edges(oracle, kind):
+    """Half rows equal to the oracle's, order included, and full rows the same
+    pairs from both ends, where the build changes path."""
+    from protein_physics_b200.device import DeviceBatch
+    clouds = _clouds(kind)
+    b = DeviceBatch([(x, np.zeros(len(x)), np.full(len(x), 1.9), np.full(len(x), 0.1), None) for x in clouds])
+    assert kind != "two per warp" or b.natoms >= 24000
+    b.build_nl()
+    need = b.need.cpu().numpy()
+    for s, x in enumerate(clouds):
+        rp, cols, _ = b.nl_host(s, half=True)
+        ptr, ocols = oracle.nl_build(x)
+        assert np.array_equal(rp, ptr) and np.array_equal(cols, ocols), s
+        frp, fcols, _ = b.nl_host(s, half=False)
+        n = len(x)
+        I = np.repeat(np.arange(n), np.diff(ptr))
+        J = np.repeat(np.arange(n), np.diff(frp))
+        both = np.concatenate([I * n + ocols, ocols.astype(np.int64) * n + I])
+        assert np.array_equal(np.sort(J * n + fcols), np.sort(both)), s
+        keep = fcols > J  # the full row holds the half row in its order
+        assert np.array_equal(fcols[keep], ocols), s
+        assert need[s, 0] == len(fcols) and need[s, 1] == len(ocols)
