@@ -258,10 +258,9 @@ nl_order_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, cons
 //          tests bit for bit
 //   write  space from the system's counters (one atomic per row kind, which
 //          are also the entry counts), then the four rows, ballot-compacted
-// Issue and L1 latency bound it (24-28 warps per SM by registers and shared
-// memory).  The scan before this one compacted every chunk of 27 separate
+// Issue bounds it (69 % active with 28 warps per SM, 36 fit).  The scan before this one compacted every chunk of 27 separate
 // cells as it went, about 12,000 issue slots per atom at 600 neighbours.  65k
-// atoms: 1,010 -> 445 us; 48 x 4.8k atoms: 1,892 -> 978 us.  Rows sit in their system's region in any order; a row that
+// atoms: 1,010 -> 431 us; 48 x 4.8k atoms: 1,892 -> 926 us.  Rows sit in their system's region in any order; a row that
 // would overflow it is not written and raises the flag.
 constexpr int NL_STAGE = 1280;  // staged entries of a row; a longer one is scanned in FP64
 constexpr int NL_CHUNKS = 160;  // chunks of 32 candidates that hold one within reach; likewise
@@ -303,7 +302,7 @@ __device__ __forceinline__ void set_rows(const AlmaNL &nl, int i, int n, int lan
 }
 
 template <int G>
-__global__ void __launch_bounds__(NL_WARPS * 32, G == 1 ? 8 : 7)
+__global__ void __launch_bounds__(NL_WARPS * 32, 9)
 nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const uint8_t *__restrict__ mask,
                const double *__restrict__ xyz, double rcut2, const SysGrid *__restrict__ grid,
                const int32_t *__restrict__ cell_of, const int32_t *__restrict__ cell_end,
