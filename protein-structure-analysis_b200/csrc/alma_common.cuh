@@ -111,35 +111,68 @@ __device__ __forceinline__ double m_abs(double x) { return fabs(x); }
 __device__ __forceinline__ float f_sqrt(float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; }
 __device__ __forceinline__ double f_sqrt(double x) { return sqrt(x); }
 
+// LJ + hard core of a contact inside sigma (r2d < sig2), FP64: the steep
+// terms, where a clash's r^-12 would amplify the FP32 rounding of sigma
+// twelvefold.
+__device__ __forceinline__ double lj_contact(const DevParams &P, double r2d, double sig2, double sig64, double eps64) {
+    const double s2 = sig2 / r2d, s6 = s2 * s2 * s2;
+    double lj = 4.0 * sqrt(eps64) * (s6 * s6 - s6);
+    const double rc = sig64 * P.hard_frac, rc2 = rc * rc;
+    if (r2d < rc2) {
+        const double t2 = rc2 / r2d, t6 = t2 * t2 * t2, x = t6 * t6 - 1.0;
+        lj += fmin(P.hard_scale * x * x, P.hard_cap);
+    }
+    return lj;
+}
+
+// The GB function f² = r² + A exp(-r²/4A), A = a_i a_j, is r² to the last FP32
+// bit once r² >= 60 A: the second term is at most A e^-15 < 60 A 2^-25, half
+// an ulp.  With Born radii of at most 0.5 Å (born_radii's clamp) every pair
+// beyond 3.9 Å is far, all but 3-4 % of those within the cutoff.
+constexpr float GB_FAR = 60.0f;
+
+// The FP32 pair sums are written operation by operation, so that every kernel
+// that evaluates a pair rounds it the same way, whatever the compiler would
+// contract in its surroundings: K qq e^{-κr}/r and C qq/f are rounded, then
+// added; 4√εε (s¹² - s⁶) goes in with multiply-adds.
+__device__ __forceinline__ float add_screened(float dh_scale, float dh_exp, float gb_scale, float gb_rinv) {
+    return __fadd_rn(__fmul_rn(gb_scale, gb_rinv), __fmul_rn(dh_scale, dh_exp));
+}
+
+__device__ __forceinline__ float add_lj(float e, float sig, float rinv, float eps_prod) {
+    const float sr = __fmul_rn(sig, rinv), s2 = __fmul_rn(sr, sr), s6 = __fmul_rn(__fmul_rn(s2, s2), s2);
+    return __fmaf_rn(__fmul_rn(4.0f, f_sqrt(eps_prod)), __fmaf_rn(s6, s6, -s6), e);
+}
+
+// One far pair outside sigma in FP32, rinv = 1/r: the value pair_energy gives,
+// without GB's exponential, division and second root.
+__device__ __forceinline__ float pair_energy_far(const DevParams &P, float r2, float rinv, float qp, float sig,
+                                                 float eps_prod) {
+    const float r = __fmul_rn(r2, rinv);
+    const float e = add_screened(__fmul_rn(__fmul_rn((float)P.coulomb_over_epsw, qp), rinv),
+                                 __expf(__fmul_rn(-(float)P.kappa, r)), __fmul_rn((float)P.gb_coef, qp), rinv);
+    return add_lj(e, sig, rinv, eps_prod);
+}
+
 // One nonbonded pair: Debye-Hückel + GB + LJ 12-6 + smooth capped hard core.
 // r2d is the FP64 squared distance; q = qi*qj product; the caller has
 // already applied the exclusion and 12 Å tests.  FP32: the fast forms
 // above, and LJ + hard core in FP64 with the FP64 sigma / epsilon product
-// (sig64, eps64) inside sigma (the steep terms: a clash's r^-12 would
-// amplify the FP32 rounding of sigma twelvefold).
+// (sig64, eps64) inside sigma.
 template <typename R>
 __device__ __forceinline__ R pair_energy(const DevParams &P, double r2d, R qp, R sig, R eps_prod,
                                          R ai, R aj, double sig64, double eps64) {
     if constexpr (sizeof(R) == 4) {
         const float r2 = (float)r2d;
-        const float rinv = rsqrtf(r2), r = r2 * rinv;
-        const float edh = (float)P.coulomb_over_epsw * qp * rinv * __expf(-(float)P.kappa * r);
-        const float aa = ai * aj;
-        const float f2 = r2 + aa * __expf(-0.25f * __fdividef(r2, aa));
-        const float egb = (float)P.gb_coef * qp * rsqrtf(f2);
+        const float rinv = rsqrtf(r2), r = __fmul_rn(r2, rinv);
+        const float aa = __fmul_rn(ai, aj);
+        const float f2 = __fmaf_rn(aa, __expf(__fmul_rn(-0.25f, __fdividef(r2, aa))), r2);
+        const float e = add_screened(__fmul_rn(__fmul_rn((float)P.coulomb_over_epsw, qp), rinv),
+                                     __expf(__fmul_rn(-(float)P.kappa, r)), __fmul_rn((float)P.gb_coef, qp),
+                                     rsqrtf(f2));
         const double sig2 = sig64 * sig64;
-        if (r2d < sig2) {
-            const double s2 = sig2 / r2d, s6 = s2 * s2 * s2;
-            double lj = 4.0 * sqrt(eps64) * (s6 * s6 - s6);
-            const double rc = sig64 * P.hard_frac, rc2 = rc * rc;
-            if (r2d < rc2) {
-                const double t2 = rc2 / r2d, t6 = t2 * t2 * t2, x = t6 * t6 - 1.0;
-                lj += fmin(P.hard_scale * x * x, P.hard_cap);
-            }
-            return (float)((double)(edh + egb) + lj);
-        }
-        const float sr = sig * rinv, s2 = sr * sr, s6 = s2 * s2 * s2;
-        return edh + egb + 4.0f * f_sqrt(eps_prod) * (s6 * s6 - s6);
+        if (r2d < sig2) return (float)((double)e + lj_contact(P, r2d, sig2, sig64, eps64));
+        return add_lj(e, sig, rinv, eps_prod);
     }
     const R r2 = (R)r2d;
     const R r = m_sqrt(r2);
@@ -265,6 +298,25 @@ __device__ __forceinline__ double4 ld_xyz(const double *xyz, int i) {
     return *reinterpret_cast<const double4 *>(xyz + 4 * (size_t)i);
 }
 
+// Position of atom j in a kernel that does not write xyz.  WIDE: xyz starts on
+// a 32-byte boundary, and the whole position is one 256-bit load — a gather
+// of 32 rows then takes half the L1 wavefronts of two 128-bit loads, each of
+// which touches every row's sector.
+template <bool WIDE>
+__device__ __forceinline__ double4 ld_pos(const double *__restrict__ xyz, int j) {
+    if constexpr (WIDE) {
+        double4 p;
+        asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+            : "=d"(p.x), "=d"(p.y), "=d"(p.z), "=d"(p.w)
+            : "l"(xyz + 4 * (size_t)j));
+        return p;
+    } else {
+        return ld_xyz(xyz, j);
+    }
+}
+
+inline bool wide_ok(const void *p) { return ((uintptr_t)p & 31) == 0; }
+
 __device__ __forceinline__ double d2_of(double4 a, double4 b) {
     const double dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
     return dx * dx + dy * dy + dz * dz;
@@ -313,6 +365,19 @@ __device__ __forceinline__ double sasa_chunk(double sa, unsigned hits, double c,
         sa = sasa_step(sasa_step(sasa_step(sasa_step(sa, c0), c1), c2), c3);
     }
     for (; k < n; ++k) sa = sasa_step(sa, __shfl_sync(0xffffffffu, packed, k));
+    return sa;
+}
+
+// The same step for entries already packed into lanes 0..n-1 (an entry of 0
+// changes nothing: sa stays positive).
+__device__ __forceinline__ double sasa_steps(double sa, int n, double c) {
+    int k = 0;
+    for (; k + 4 <= n; k += 4) {
+        const double c0 = __shfl_sync(0xffffffffu, c, k), c1 = __shfl_sync(0xffffffffu, c, k + 1);
+        const double c2 = __shfl_sync(0xffffffffu, c, k + 2), c3 = __shfl_sync(0xffffffffu, c, k + 3);
+        sa = sasa_step(sasa_step(sasa_step(sasa_step(sa, c0), c1), c2), c3);
+    }
+    for (; k < n; ++k) sa = sasa_step(sa, __shfl_sync(0xffffffffu, c, k));
     return sa;
 }
 

@@ -22,7 +22,7 @@ namespace alma {
 
 namespace cg = cooperative_groups;
 
-template <typename R>
+template <typename R, bool WIDE>
 __global__ void born_kernel(int natoms, const int32_t *__restrict__ atom_off, int nsys, const uint8_t *__restrict__ mask,
                             const double *__restrict__ xyz, const float *__restrict__ prm,
                             const double *__restrict__ prm64, const int64_t *__restrict__ full_ptr,
@@ -32,26 +32,28 @@ __global__ void born_kernel(int natoms, const int32_t *__restrict__ atom_off, in
     const int lane = threadIdx.x & 31;
     if (i >= natoms) return;
     if (mask && !mask[sys_of_atom(atom_off, nsys, i)]) return;
-    born_atom<R>(i, lane, xyz, prm, prm64, full_ptr, full_len, full_cols, born);
+    born_atom<R, WIDE>(i, lane, xyz, prm, prm64, full_ptr, full_len, full_cols, born);
 }
 
 // Warp per atom: pair energy and SASA of row i.  atom_e[2*i] = pair sum of
-// row i, atom_e[2*i+1] = gamma * max(0, sa_i).  Held to 64 registers (four
-// 256-thread blocks per SM): the row gathers are latency bound and need the
-// resident warps.
-template <typename R>
-__global__ void __launch_bounds__(256, 4) pair_sasa_kernel(DevParams P, int natoms, const int32_t *__restrict__ atom_off, int nsys,
+// row i, atom_e[2*i+1] = gamma * max(0, sa_i).  Five 256-thread blocks per SM (48
+// registers): the row gathers are latency bound and need the resident warps
+// (65k atoms: 216 us with four blocks, 196 with five, 203 with six).
+template <typename R, bool WIDE>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 4) pair_sasa_kernel(DevParams P, int natoms, const int32_t *__restrict__ atom_off, int nsys,
                                  const uint8_t *__restrict__ mask, const double *__restrict__ xyz,
                                  const float *__restrict__ prm,
                                  const double *__restrict__ prm64, const double *__restrict__ born,
                                  const int64_t *__restrict__ half_ptr, const int32_t *__restrict__ half_len,
                                  const uint32_t *__restrict__ half_cols, int use_excl, double *__restrict__ atom_e,
                                  double *__restrict__ sasa_out) {
+    __shared__ PairBuf buf[8];
     const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (i >= natoms) return;
     if (mask && !mask[sys_of_atom(atom_off, nsys, i)]) return;
-    pair_sasa_atom<R>(P, i, lane, xyz, prm, prm64, born, half_ptr, half_len, half_cols, use_excl, atom_e, sasa_out);
+    pair_sasa_atom<R, WIDE>(P, i, lane, xyz, prm, prm64, born, half_ptr, half_len, half_cols, use_excl,
+                            buf[threadIdx.x >> 5], atom_e, sasa_out);
 }
 
 // One cluster of 8 CTAs per system: the atoms' and records' terms strided over
@@ -133,10 +135,11 @@ extern "C" int alma_born_radii(const AlmaBatch *b, const AlmaNL *nl, const AlmaP
     if (b->natoms == 0) return ALMA_OK;
     cudaStream_t st = (cudaStream_t)stream;
     const int wpb = 8, nb = (b->natoms + wpb - 1) / wpb;
-    if (prec == ALMA_PREC_FP64)
-        born_kernel<double><<<nb, wpb * 32, 0, st>>>(b->natoms, b->atom_off, b->nsys, sys_mask, b->xyz, b->prm, b->prm64, nl->full_ptr, nl->full_len, nl->full_cols, b->born);
-    else
-        born_kernel<float><<<nb, wpb * 32, 0, st>>>(b->natoms, b->atom_off, b->nsys, sys_mask, b->xyz, b->prm, b->prm64, nl->full_ptr, nl->full_len, nl->full_cols, b->born);
+    const bool wide = wide_ok(b->xyz);
+    auto kfn = prec == ALMA_PREC_FP64 ? (wide ? born_kernel<double, true> : born_kernel<double, false>)
+                                      : (wide ? born_kernel<float, true> : born_kernel<float, false>);
+    kfn<<<nb, wpb * 32, 0, st>>>(b->natoms, b->atom_off, b->nsys, sys_mask, b->xyz, b->prm, b->prm64, nl->full_ptr,
+                                 nl->full_len, nl->full_cols, b->born);
     ALMA_LAUNCH_CHECK("alma_born_radii");
     return ALMA_OK;
 }
@@ -152,12 +155,11 @@ extern "C" int alma_energy(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *
     if (b->natoms > 0) {
         const int wpb = 8, nb = (b->natoms + wpb - 1) / wpb;
         const int use_excl = t != nullptr;
-        if (prec == ALMA_PREC_FP64)
-            pair_sasa_kernel<double><<<nb, wpb * 32, 0, st>>>(P, b->natoms, b->atom_off, b->nsys, sys_mask, b->xyz, b->prm, b->prm64, b->born,
-                                                              nl->half_ptr, nl->half_len, nl->half_cols, use_excl, atom_e, b->sasa);
-        else
-            pair_sasa_kernel<float><<<nb, wpb * 32, 0, st>>>(P, b->natoms, b->atom_off, b->nsys, sys_mask, b->xyz, b->prm, b->prm64, b->born,
-                                                             nl->half_ptr, nl->half_len, nl->half_cols, use_excl, atom_e, b->sasa);
+        const bool wide = wide_ok(b->xyz);
+        auto kfn = prec == ALMA_PREC_FP64 ? (wide ? pair_sasa_kernel<double, true> : pair_sasa_kernel<double, false>)
+                                          : (wide ? pair_sasa_kernel<float, true> : pair_sasa_kernel<float, false>);
+        kfn<<<nb, wpb * 32, 0, st>>>(P, b->natoms, b->atom_off, b->nsys, sys_mask, b->xyz, b->prm, b->prm64, b->born,
+                                     nl->half_ptr, nl->half_len, nl->half_cols, use_excl, atom_e, b->sasa);
     }
     AlmaTopo tt;
     if (t) tt = *t;

@@ -194,7 +194,7 @@ __device__ void team_minmax3(const Team<CL> &T, double (&lo)[3], double (&hi)[3]
 // host rebuild, which grows the regions.  E: the fresh total energy.
 template <typename R, int CL>
 __device__ bool team_rebuild(const MoveCtx &C, const MCConfigDev &cfg, int s, const Team<CL> &T, double *sm,
-                             double *rsm, double *rpart, int64_t *ssm, double &E) {
+                             double *rsm, double *rpart, int64_t *ssm, PairBuf *pair_buf, double &E) {
     const RebuildWS &ws = cfg.rw;
     const AlmaBatch &b = C.b;
     const AlmaNL &nl = C.nl;
@@ -324,7 +324,7 @@ __device__ bool team_rebuild(const MoveCtx &C, const MCConfigDev &cfg, int s, co
     T.sync();
     for (int i = a0 + wid; i < a1; i += nw)
         pair_sasa_atom<R>(C.P, i, lane, b.xyz, b.prm, b.prm64, b.born, nl.half_ptr, nl.half_len, nl.half_cols,
-                          ep != nullptr, ws.atom_e, b.sasa);
+                          ep != nullptr, pair_buf[threadIdx.x >> 5], ws.atom_e, b.sasa);
     T.sync();
     double v[4] = {0.0, 0.0, 0.0, 0.0};
     for (int i = a0 + tid; i < a1; i += nthr) {
@@ -355,7 +355,11 @@ __global__ void __launch_bounds__(NT, 512 / NT) mc_kernel(MoveCtx C, MCConfigDev
     __shared__ MoveDesc M;
     __shared__ double sm[128];
     __shared__ double part[8];
-    __shared__ CrossCand cq[(NT / 32) * CROSS_BUF];
+    __shared__ union {  // per warp; a rebuild runs between proposals
+        CrossCand cross[(NT / 32) * CROSS_BUF];
+        PairBuf pair[NT / 32];
+    } wb;
+    CrossCand *cq = wb.cross;
     __shared__ AlmaChainState S;
     __shared__ double u[6];
     __shared__ int did_move, accept;
@@ -384,7 +388,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) mc_kernel(MoveCtx C, MCConfigDev
     while (S.step < step_limit) {
         if (S.need_rebuild) {  // drifted: rebuild this chain in place, or stop for the host
             double E = 0.0;
-            if (!cfg.rw.ccount || !C.nl.ref_xyz || !team_rebuild<R, CL>(C, cfg, s, T, sm, rsm, rpart, ssm, E)) break;
+            if (!cfg.rw.ccount || !C.nl.ref_xyz || !team_rebuild<R, CL>(C, cfg, s, T, sm, rsm, rpart, ssm, wb.pair, E)) break;
             if (threadIdx.x == 0) {
                 S.energy = E;
                 S.n_rebuild++;
