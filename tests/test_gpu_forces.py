@@ -160,3 +160,37 @@ def test_evaluate_graph_equals_eager(precision):
     xg = x.clone().requires_grad_()
     model(xg).sum().backward()
     assert torch.equal(xg.grad, ge[:n, :3])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("spacing,n", [(1.5, 8), (2.2, 7), (9.0, 3)])
+def test_forces_of_jittered_lattices(precision, spacing, n, oracle):
+    """Energy and forces where the kernels' packed lists change path: rows with
+    more SASA entries than the list holds (1.5 Å), several batches of near
+    pairs (2.2 Å), none at all (9 Å); positions on a 32-byte boundary or not
+    (one or two loads) give the same bits."""
+    from torch_energy import TorchEnergy
+    from protein_physics_b200.device import DeviceBatch
+    rng = np.random.default_rng(17)
+    k = np.arange(n, dtype=np.float64) * spacing
+    x = np.stack(np.meshgrid(k, k, k, indexing="ij"), -1).reshape(-1, 3) + rng.uniform(-0.2, 0.2, (n ** 3, 3))
+    m = len(x)
+    q, r = rng.normal(0, 0.4, m), rng.choice([0.6, 1.487, 1.908], m)
+    eps = rng.uniform(0.01, 0.2, m)
+    ptr, cols = oracle.nl_build(x)
+    E, gt = TorchEnergy(q, r, eps, ptr, cols).energy_and_grad(x)
+    out = []
+    for aligned in (True, False):
+        b = DeviceBatch([(x, q, r, eps, None)], precision=precision)
+        if not aligned:
+            buf = torch.zeros(4 * m + 2, dtype=torch.float64, device="cuda")
+            buf[2:].copy_(b.xyz.reshape(-1))
+            b.xyz, b._batch_s = buf[2:].view(m, 4), None
+        assert (b.xyz.data_ptr() % 32 == 0) == aligned
+        terms, grad = b.evaluate()
+        out.append((terms.cpu().numpy(), grad.cpu().numpy()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    # the module's bars, relative to the largest force of these clashing systems
+    scale = np.abs(gt).max()
+    assert np.abs(out[0][1][:, :3] - gt).max() <= (1e-9 if precision == "fp64" else 2e-4) * max(scale, 1.0)
+    assert abs(out[0][0][0, 4] - E) <= (1e-10 if precision == "fp64" else 1e-6) * max(abs(E), 1.0)
