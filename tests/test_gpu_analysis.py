@@ -48,3 +48,15 @@ def test_device_tensor_in_device_tensor_out():
     assert analysis.compute_mean_dist_matrix(np.zeros((0, 3, 3))).shape == (3, 3)
     with pytest.raises(ValueError):
         analysis.compute_mean_dist_matrix(np.zeros((3, 3)))
+
+
+@pytest.mark.parametrize("n_snaps,n_ca", [(8, 16), (9, 31), (16, 32), (17, 49), (1, 97), (3, 1)])
+def test_matrices_at_tile_and_stage_edges(n_snaps, n_ca):
+    """Residue counts around the tile's 32 rows and 16 columns, snapshots
+    around the eight staged at a time."""
+    from protein_physics_b200 import analysis
+    c = np.random.default_rng(n_ca).normal(size=(n_snaps, n_ca, 3)) * 12.0
+    np.testing.assert_allclose(analysis.compute_mean_dist_matrix(c), _numpy_mean(c), rtol=1e-12, atol=1e-12)
+    f = (np.sqrt(((c[:, :, None, :] - c[:, None, :, :]) ** 2).sum(-1)) < 8.0).mean(0)
+    np.fill_diagonal(f, 0.0)
+    np.testing.assert_allclose(analysis.compute_contact_freq_matrix(c, 8.0), f, rtol=1e-15, atol=1e-15)
