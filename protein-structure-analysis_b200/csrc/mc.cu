@@ -816,16 +816,12 @@ extern "C" int alma_mc_run(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *
     d.reach_pad = 2.0 * p->probe_r + 2.0 * sqrt(p->half_skin2) + 1e-6;  // as alma_nl_build
     d.rw = carve_rebuild(cfg->rebuild_ws, b->natoms, b->nsys);
     cudaStream_t st = (cudaStream_t)stream;
-    // Threads per system: 512 when the batch fits one CTA per SM, else 256
-    // (two CTAs per SM), so every chain of a persistent launch is resident.
+    // Threads per CTA: 512 unless the caller asks for 256.  One 512-thread CTA
+    // fills an SM (128 registers); 256 threads keep two chains resident per SM,
+    // but each takes twice as long and the longest one then ends the launch
+    // (256 chains of 50-600 residues: 407 ms against 783).
     // cluster_size CTAs cooperate on each system (1, 2, 4, 8 or 16).
-    int nt = cfg->threads_per_system;
-    if (nt == 0) {
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        nt = nl_sys <= sms ? 512 : 256;
-    }
+    const int nt = cfg->threads_per_system == 0 ? 512 : cfg->threads_per_system;
     const int cl = cfg->cluster_size <= 0 ? 1 : cfg->cluster_size;
     if (nt != 256 && nt != 512) return alma_set_error(ALMA_EINVAL, "alma_mc_run: threads_per_system must be 0, 256 or 512");
     if (cl != 1 && cl != 2 && cl != 4 && cl != 8 && cl != 16)

@@ -68,3 +68,18 @@ def test_tail_plan_leaves_a_small_batch_its_own_shape_until_a_chain_is_done():
     steps[3] = 100
     assert MCRunner._tail_plan(R, _states(steps), 100)[1:] == (15,) + auto_shape(15, 148)
 
+
+
+def test_auto_shape_of_queued_systems_balances_the_longest_chain():
+    """More systems than half the SMs: the cluster takes the largest system
+    below 0.4 of the work per SM; fewer keep one cluster each."""
+    rng = np.random.default_rng(2)
+    for n in (75, 148, 256, 1000):
+        for sizes in (np.full(n, 5000), rng.integers(800, 10000, n), np.r_[np.full(n - 1, 500), 60000]):
+            cl, k = auto_shape(n, 148, sizes)
+            share = sizes.sum() / 148
+            assert cl in (1, 2, 4, 8) and k == 1
+            assert cl == 8 or sizes.max() / cl <= 0.4 * share
+            assert cl == 1 or sizes.max() / (cl // 2) > 0.4 * share
+    assert auto_shape(74, 148, np.full(74, 5000)) == (2, 1)
+    assert auto_shape(256, 148, np.linspace(800, 9800, 256)) == (4, 1)
