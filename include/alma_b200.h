@@ -405,7 +405,7 @@ typedef struct {
     double fixed_delta;       /* > 0: angles ~ U(-fixed_delta, fixed_delta)  */
     const int32_t *moveset_off;   /* optional [nsys+1] device: torsion moves */
     const int32_t *moveset;       /* drawn from these local rot-bond indices */
-    int32_t threads_per_system;   /* CTA size 256 or 512; 0 = 512            */
+    int32_t threads_per_system;   /* CTA size 256 or 512; 0 = 512 or 1024     */
     int32_t cluster_size;         /* CTAs per system (1,2,4,8,16; 0 = 1): a  */
                                   /* thread-block cluster shares a proposal  */
     int32_t spec_teams;           /* teams (clusters) per system, 0/1 = one: */

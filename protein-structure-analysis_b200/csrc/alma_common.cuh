@@ -111,6 +111,14 @@ __device__ __forceinline__ double m_abs(double x) { return fabs(x); }
 __device__ __forceinline__ float f_sqrt(float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; }
 __device__ __forceinline__ double f_sqrt(double x) { return sqrt(x); }
 
+// 1/x in FP64 from an FP32 estimate y0 of it (within a few 2^-22) and one
+// Newton step, y1 = y0 (2 - x y0): relative error below 2^-40.  For quotients
+// that are rounded to FP32 next, or multiply an FP32 factor.
+__device__ __forceinline__ double recip_from(double x, float y0) {
+    const double y = (double)y0;
+    return fma(y, fma(-x, y, 1.0), y);
+}
+
 // LJ + hard core of a contact inside sigma (r2d < sig2), FP64: the steep
 // terms, where a clash's r^-12 would amplify the FP32 rounding of sigma
 // twelvefold.
@@ -205,20 +213,16 @@ __device__ __forceinline__ double m_log1p(double x) { return log1p(x); }
 // LJ 12-6 + capped hard core of one pair (r2 in FP64).  Inside sigma the
 // terms grow steeply and are evaluated in FP64 with FP64 sigma and
 // epsilon (sig64 = R*_i + R*_j, eps64 = eps_i eps_j); outside, in
-// precision R.
+// precision R (FP32: s² from an FP64 quotient, rinv = 1/r).
 template <typename R>
 __device__ __forceinline__ double lj_hard(const DevParams &P, double r2, R sig, R eps_prod, double sig64,
-                                          double eps64) {
+                                          double eps64, R rinv) {
     const double sig2 = sig64 * sig64;
-    if (r2 < sig2) {
-        const double s2 = sig2 / r2, s6 = s2 * s2 * s2;
-        double E = 4.0 * sqrt(eps64) * (s6 * s6 - s6);
-        const double rc = sig64 * P.hard_frac, rc2 = rc * rc;
-        if (r2 < rc2) {
-            const double t2 = rc2 / r2, t6 = t2 * t2 * t2, x = t6 * t6 - 1.0;
-            E += fmin(P.hard_scale * x * x, P.hard_cap);
-        }
-        return E;
+    if (r2 < sig2) return lj_contact(P, r2, sig2, sig64, eps64);
+    if constexpr (sizeof(R) == 4) {
+        const float s2 = (float)__dmul_rn(sig2, recip_from(r2, __fmul_rn(rinv, rinv)));
+        const float s6 = __fmul_rn(__fmul_rn(s2, s2), s2);
+        return (double)__fmul_rn(__fmul_rn(4.0f, sqrtf(eps_prod)), __fmaf_rn(s6, s6, -s6));
     }
     const R s2 = (R)(sig2 / r2);
     const R s6 = s2 * s2 * s2;
@@ -244,14 +248,17 @@ __device__ __forceinline__ double pair_delta(const DevParams &P, double r2o, dou
         const float kap = (float)P.kappa;
         const float gdo = (float)P.coulomb_over_epsw * qp * rio * __expf(-kap * ro);
         const float ddh = gdo * expm1f(-kap * dr - log1pf(dr * rio));
-        const float xo = aao * __expf(-0.25f * __fdividef(ro2, aao));
-        const float xn = aan * __expf(-0.25f * __fdividef(rn2, aan));
+        float xo = 0.0f, xn = 0.0f;  // below the last bit of f² for far pairs (GB_FAR)
+        if (ro2 < GB_FAR * aao || rn2 < GB_FAR * aan) {
+            xo = aao * __expf(-0.25f * __fdividef(ro2, aao));
+            xn = aan * __expf(-0.25f * __fdividef(rn2, aan));
+        }
         const float fo2 = ro2 + xo, fn2 = rn2 + xn;
         const float fo = fo2 * rsqrtf(fo2), fn = fn2 * rsqrtf(fn2);
         const float num = (float)(-d2) + (xo - xn);
         const float dgb = (float)P.gb_coef * qp * __fdividef(num, fo * fn * (fo + fn));
         return (double)ddh + (double)dgb +
-               (lj_hard<float>(P, r2n, sig, eps_prod, sig64, eps64) - lj_hard<float>(P, r2o, sig, eps_prod, sig64, eps64));
+               (lj_hard<float>(P, r2n, sig, eps_prod, sig64, eps64, rin) - lj_hard<float>(P, r2o, sig, eps_prod, sig64, eps64, rio));
     }
     const double d2 = r2n - r2o;
     const R ro2 = (R)r2o, rn2 = (R)r2n;
@@ -265,7 +272,7 @@ __device__ __forceinline__ double pair_delta(const DevParams &P, double r2o, dou
     const R num = (R)(-d2) + (xo - xn);
     const R dgb = (R)P.gb_coef * qp * num / (fo * fn * (fo + fn));
     return (double)ddh + (double)dgb +
-           (lj_hard<R>(P, r2n, sig, eps_prod, sig64, eps64) - lj_hard<R>(P, r2o, sig, eps_prod, sig64, eps64));
+           (lj_hard<R>(P, r2n, sig, eps_prod, sig64, eps64, (R)0) - lj_hard<R>(P, r2o, sig, eps_prod, sig64, eps64, (R)0));
 }
 
 // HCT descreening integral of atom j (radius rj) on atom i (radius ri).
@@ -338,14 +345,11 @@ __device__ __forceinline__ double warp_max(double v) {
 }
 
 // ---------------------------------------------------------------------------
-// SASA cap recurrence (physics_engine.cpp:2068-2083) over a 32-entry chunk
-// of a row: sa -= min(0.85 sa, c_l) for every lane l set in `hits`, in lane
-// (= row) order.  The hit values are first packed into lanes 0..n-1 (one
-// shuffle from the position of each lane's set bit), then read back by
-// index in groups of four: those shuffles do not depend on sa, so they
-// issue ahead of the dependent FP64 chain instead of one round trip per
-// entry.  The arithmetic and its order are those of the entry-by-entry
-// loop, so the result is the same to the bit.
+// SASA cap recurrence (physics_engine.cpp:2068-2083): sa -= min(0.85 sa, c) for
+// each entry within reach, in row order.  The values wait packed in lanes
+// 0..n-1 and are read back by index in groups of four: those shuffles do not
+// depend on sa, so they issue ahead of the dependent FP64 chain instead of one
+// round trip per entry.  An entry of 0 changes nothing (sa stays positive).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double sasa_pack(unsigned hits, double c, int lane) {
     const int src = lane < __popc(hits) ? (int)__fns(hits, 0, lane + 1) : lane;
@@ -354,22 +358,6 @@ __device__ __forceinline__ double sasa_pack(unsigned hits, double c, int lane) {
 
 __device__ __forceinline__ double sasa_step(double sa, double c) { return sa - fmin(sa * 0.85, c); }
 
-__device__ __forceinline__ double sasa_chunk(double sa, unsigned hits, double c, int lane) {
-    const int n = __popc(hits);
-    if (n == 0) return sa;
-    const double packed = sasa_pack(hits, c, lane);
-    int k = 0;
-    for (; k + 4 <= n; k += 4) {
-        const double c0 = __shfl_sync(0xffffffffu, packed, k), c1 = __shfl_sync(0xffffffffu, packed, k + 1);
-        const double c2 = __shfl_sync(0xffffffffu, packed, k + 2), c3 = __shfl_sync(0xffffffffu, packed, k + 3);
-        sa = sasa_step(sasa_step(sasa_step(sasa_step(sa, c0), c1), c2), c3);
-    }
-    for (; k < n; ++k) sa = sasa_step(sa, __shfl_sync(0xffffffffu, packed, k));
-    return sa;
-}
-
-// The same step for entries already packed into lanes 0..n-1 (an entry of 0
-// changes nothing: sa stays positive).
 __device__ __forceinline__ double sasa_steps(double sa, int n, double c) {
     int k = 0;
     for (; k + 4 <= n; k += 4) {
@@ -379,24 +367,6 @@ __device__ __forceinline__ double sasa_steps(double sa, int n, double c) {
     }
     for (; k < n; ++k) sa = sasa_step(sa, __shfl_sync(0xffffffffu, c, k));
     return sa;
-}
-
-// Two independent recurrences (old and new geometry) over the same chunk,
-// interleaved.
-__device__ __forceinline__ void sasa_chunk2(double &sa_a, unsigned hits_a, double c_a, double &sa_b,
-                                            unsigned hits_b, double c_b, int lane) {
-    const int na = __popc(hits_a), nb = __popc(hits_b);
-    const double pa = sasa_pack(hits_a, c_a, lane), pb = sasa_pack(hits_b, c_b, lane);
-    const int n = na < nb ? na : nb;
-    int k = 0;
-    for (; k + 2 <= n; k += 2) {
-        const double a0 = __shfl_sync(0xffffffffu, pa, k), a1 = __shfl_sync(0xffffffffu, pa, k + 1);
-        const double b0 = __shfl_sync(0xffffffffu, pb, k), b1 = __shfl_sync(0xffffffffu, pb, k + 1);
-        sa_a = sasa_step(sasa_step(sa_a, a0), a1);
-        sa_b = sasa_step(sasa_step(sa_b, b0), b1);
-    }
-    for (int q = k; q < na; ++q) sa_a = sasa_step(sa_a, __shfl_sync(0xffffffffu, pa, q));
-    for (int q = k; q < nb; ++q) sa_b = sasa_step(sa_b, __shfl_sync(0xffffffffu, pb, q));
 }
 
 // Block-wide sum; every thread gets the result.  smem: >= 32 doubles.

@@ -103,14 +103,6 @@ __device__ __forceinline__ double grad_contact(const DevParams &P, double r2d, d
     return f;
 }
 
-// 1/x in FP64 from an FP32 estimate y0 of it (within a few 2^-22) and one
-// Newton step, y1 = y0 (2 - x y0): relative error below 2^-40.  For quotients
-// that are rounded to FP32 next, or multiply an FP32 factor.
-__device__ __forceinline__ double recip_from(double x, float y0) {
-    const double y = (double)y0;
-    return fma(y, fma(-x, y, 1.0), y);
-}
-
 // LJ outside sigma: s² in FP64, the powers in R.
 template <typename R>
 __device__ __forceinline__ double grad_lj(double r2d, double sig2, R eps_prod) {

@@ -350,16 +350,13 @@ __device__ bool team_rebuild(const MoveCtx &C, const MCConfigDev &cfg, int s, co
 // and decisions (the ΔE totals are bit-identical in every CTA); rank 0
 // writes the state back.
 template <typename R, int NT, int CL>
-__global__ void __launch_bounds__(NT, 512 / NT) mc_kernel(MoveCtx C, MCConfigDev cfg,
+__global__ void __launch_bounds__(NT) mc_kernel(MoveCtx C, MCConfigDev cfg,
                                                           AlmaChainState *__restrict__ states, int64_t step_limit) {
     __shared__ MoveDesc M;
     __shared__ double sm[128];
     __shared__ double part[8];
-    __shared__ union {  // per warp; a rebuild runs between proposals
-        CrossCand cross[(NT / 32) * CROSS_BUF];
-        PairBuf pair[NT / 32];
-    } wb;
-    CrossCand *cq = wb.cross;
+    extern __shared__ __align__(16) unsigned char warp_smem[];  // a buffer per warp; a rebuild runs between proposals
+    CrossCand *cq = reinterpret_cast<CrossCand *>(warp_smem);
     __shared__ AlmaChainState S;
     __shared__ double u[6];
     __shared__ int did_move, accept;
@@ -388,7 +385,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) mc_kernel(MoveCtx C, MCConfigDev
     while (S.step < step_limit) {
         if (S.need_rebuild) {  // drifted: rebuild this chain in place, or stop for the host
             double E = 0.0;
-            if (!cfg.rw.ccount || !C.nl.ref_xyz || !team_rebuild<R, CL>(C, cfg, s, T, sm, rsm, rpart, ssm, wb.pair, E)) break;
+            if (!cfg.rw.ccount || !C.nl.ref_xyz || !team_rebuild<R, CL>(C, cfg, s, T, sm, rsm, rpart, ssm, reinterpret_cast<PairBuf *>(warp_smem), E)) break;
             if (threadIdx.x == 0) {
                 S.energy = E;
                 S.n_rebuild++;
@@ -438,22 +435,34 @@ __global__ void __launch_bounds__(NT, 512 / NT) mc_kernel(MoveCtx C, MCConfigDev
     if (threadIdx.x == 0 && T.rank == 0) states[s] = S;
 }
 
+// Dynamic shared memory of the MC kernels: per warp, the cross-pair buffer of a
+// proposal or the pair buffer of a rebuild.
+static size_t warp_smem_bytes(int nt) {
+    const size_t cross = sizeof(CrossCand) * CROSS_BUF, pair = sizeof(PairBuf);
+    return (size_t)(nt / 32) * (cross > pair ? cross : pair);
+}
+
 template <typename R, int NT, int CL>
 static cudaError_t launch_mc(const MoveCtx &C, const MCConfigDev &d, AlmaChainState *states, int64_t step_limit,
-                             int nsys, cudaStream_t st) {
+                             int nsys, int nt, cudaStream_t st) {
+    auto kfn = mc_kernel<R, NT, CL>;
+    const size_t smem = warp_smem_bytes(nt);
+    if (NT > 512) {  // past the 48 KB that need no opt-in
+        cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
     if constexpr (CL == 1) {
-        mc_kernel<R, NT, 1><<<nsys, NT, 0, st>>>(C, d, states, step_limit);
+        kfn<<<nsys, nt, smem, st>>>(C, d, states, step_limit);
         return cudaGetLastError();
     } else {
-        auto kfn = mc_kernel<R, NT, CL>;
         if (CL > 8) {
             cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             if (e != cudaSuccess) return e;
         }
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(nsys * CL), 1, 1);
-        cfg.blockDim = dim3(NT, 1, 1);
-        cfg.dynamicSmemBytes = 0;
+        cfg.blockDim = dim3((unsigned)nt, 1, 1);
+        cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -569,13 +578,14 @@ __global__ void spec_wait_selftest_kernel(SpecRound *Rd, uint32_t *status, int32
 }
 
 template <typename R, int NT, int CL>
-__global__ void __launch_bounds__(NT, 512 / NT)
+__global__ void __launch_bounds__(NT)
 mc_spec_kernel(MoveCtx C, MCConfigDev cfg, AlmaChainState *__restrict__ states, int64_t step_limit, int teams,
                size_t team_stride, SpecRound *__restrict__ rounds) {
     __shared__ MoveDesc M;
     __shared__ double sm[128];
     __shared__ double part[8];
-    __shared__ CrossCand cq[(NT / 32) * CROSS_BUF];
+    extern __shared__ __align__(16) unsigned char warp_smem[];  // a buffer per warp
+    CrossCand *cq = reinterpret_cast<CrossCand *>(warp_smem);
     __shared__ AlmaChainState S;
     __shared__ double u[6];
     __shared__ int did_move, acc_sh, a_sh, abort_sh;
@@ -691,13 +701,18 @@ mc_spec_kernel(MoveCtx C, MCConfigDev cfg, AlmaChainState *__restrict__ states, 
 
 template <typename R, int NT, int CL>
 static cudaError_t launch_mc_spec(const MoveCtx &C, const MCConfigDev &d, AlmaChainState *states, int64_t step_limit,
-                                  int nsys, int teams, size_t team_stride, SpecRound *rounds, cudaStream_t st,
-                                  bool *fits) {
+                                  int nsys, int nt, int teams, size_t team_stride, SpecRound *rounds,
+                                  cudaStream_t st, bool *fits) {
     auto kfn = mc_spec_kernel<R, NT, CL>;
+    const size_t smem = warp_smem_bytes(nt);
+    if (NT > 512) {
+        cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(nsys * teams * CL), 1, 1);
-    cfg.blockDim = dim3(NT, 1, 1);
-    cfg.dynamicSmemBytes = 0;
+    cfg.blockDim = dim3((unsigned)nt, 1, 1);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -816,14 +831,20 @@ extern "C" int alma_mc_run(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *
     d.reach_pad = 2.0 * p->probe_r + 2.0 * sqrt(p->half_skin2) + 1e-6;  // as alma_nl_build
     d.rw = carve_rebuild(cfg->rebuild_ws, b->natoms, b->nsys);
     cudaStream_t st = (cudaStream_t)stream;
-    // Threads per CTA: 512 unless the caller asks for 256.  One 512-thread CTA
-    // fills an SM (128 registers); 256 threads keep two chains resident per SM,
-    // but each takes twice as long and the longest one then ends the launch
-    // (256 chains of 50-600 residues: 407 ms against 783).
-    // cluster_size CTAs cooperate on each system (1, 2, 4, 8 or 16).
-    const int nt = cfg->threads_per_system == 0 ? 512 : cfg->threads_per_system;
     const int cl = cfg->cluster_size <= 0 ? 1 : cfg->cluster_size;
-    if (nt != 256 && nt != 512) return alma_set_error(ALMA_EINVAL, "alma_mc_run: threads_per_system must be 0, 256 or 512");
+    // cluster_size CTAs cooperate on each system (1, 2, 4, 8 or 16), one CTA
+    // per SM.  Threads per CTA: the caller's choice, or by size.  1,024 at 64
+    // registers hide the latency of the row scans better than 512 at 128, in
+    // spite of some spilled registers, where an average system has an atom for
+    // every four threads or more (256 chains of 50-600 residues on 4-CTA
+    // clusters: 126 ms for 50 proposals against 159; one chain of 4.9k atoms,
+    // 16 CTAs and 4 teams: 60 us a proposal against 63); with less the barriers
+    // of twice the warps cost more than that (1.1k atoms on 16 CTAs: 28 against
+    // 26).  FP64 pair terms need the registers.
+    int nt = cfg->threads_per_system;
+    if (nt != 0 && nt != 256 && nt != 512)
+        return alma_set_error(ALMA_EINVAL, "alma_mc_run: threads_per_system must be 0, 256 or 512");
+    if (nt == 0) nt = prec != ALMA_PREC_FP64 && (int64_t)b->natoms >= (int64_t)256 * cl * b->nsys ? 1024 : 512;
     if (cl != 1 && cl != 2 && cl != 4 && cl != 8 && cl != 16)
         return alma_set_error(ALMA_EINVAL, "alma_mc_run: cluster_size must be 1, 2, 4, 8 or 16");
     const int teams = cfg->spec_teams <= 1 ? 1 : cfg->spec_teams;
@@ -836,16 +857,16 @@ extern "C" int alma_mc_run(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *
         bool fits = true;
 #define ALMA_SPEC_CASE(R, NT)                                                                                   \
     switch (cl) {                                                                                               \
-        case 1: e = launch_mc_spec<R, NT, 1>(C, d, states, step_limit, nl_sys, teams, stride, rounds, st, &fits); break;   \
-        case 2: e = launch_mc_spec<R, NT, 2>(C, d, states, step_limit, nl_sys, teams, stride, rounds, st, &fits); break;   \
-        case 4: e = launch_mc_spec<R, NT, 4>(C, d, states, step_limit, nl_sys, teams, stride, rounds, st, &fits); break;   \
-        case 8: e = launch_mc_spec<R, NT, 8>(C, d, states, step_limit, nl_sys, teams, stride, rounds, st, &fits); break;   \
-        default: e = launch_mc_spec<R, NT, 16>(C, d, states, step_limit, nl_sys, teams, stride, rounds, st, &fits); break; \
+        case 1: e = launch_mc_spec<R, NT, 1>(C, d, states, step_limit, nl_sys, nt, teams, stride, rounds, st, &fits); break;   \
+        case 2: e = launch_mc_spec<R, NT, 2>(C, d, states, step_limit, nl_sys, nt, teams, stride, rounds, st, &fits); break;   \
+        case 4: e = launch_mc_spec<R, NT, 4>(C, d, states, step_limit, nl_sys, nt, teams, stride, rounds, st, &fits); break;   \
+        case 8: e = launch_mc_spec<R, NT, 8>(C, d, states, step_limit, nl_sys, nt, teams, stride, rounds, st, &fits); break;   \
+        default: e = launch_mc_spec<R, NT, 16>(C, d, states, step_limit, nl_sys, nt, teams, stride, rounds, st, &fits); break; \
     }
         if (prec == ALMA_PREC_FP64) {
-            if (nt == 512) { ALMA_SPEC_CASE(double, 512) } else { ALMA_SPEC_CASE(double, 256) }
+            if (nt <= 512) { ALMA_SPEC_CASE(double, 512) } else { ALMA_SPEC_CASE(double, 1024) }
         } else {
-            if (nt == 512) { ALMA_SPEC_CASE(float, 512) } else { ALMA_SPEC_CASE(float, 256) }
+            if (nt <= 512) { ALMA_SPEC_CASE(float, 512) } else { ALMA_SPEC_CASE(float, 1024) }
         }
 #undef ALMA_SPEC_CASE
         if (e != cudaSuccess) return alma_cuda_error(e, "alma_mc_run launch");
@@ -862,16 +883,16 @@ extern "C" int alma_mc_run(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *
     }
 #define ALMA_MC_CASE(R, NT)                                                              \
     switch (cl) {                                                                        \
-        case 1: e = launch_mc<R, NT, 1>(C, d, states, step_limit, nl_sys, st); break;   \
-        case 2: e = launch_mc<R, NT, 2>(C, d, states, step_limit, nl_sys, st); break;   \
-        case 4: e = launch_mc<R, NT, 4>(C, d, states, step_limit, nl_sys, st); break;   \
-        case 8: e = launch_mc<R, NT, 8>(C, d, states, step_limit, nl_sys, st); break;   \
-        default: e = launch_mc<R, NT, 16>(C, d, states, step_limit, nl_sys, st); break; \
+        case 1: e = launch_mc<R, NT, 1>(C, d, states, step_limit, nl_sys, nt, st); break;   \
+        case 2: e = launch_mc<R, NT, 2>(C, d, states, step_limit, nl_sys, nt, st); break;   \
+        case 4: e = launch_mc<R, NT, 4>(C, d, states, step_limit, nl_sys, nt, st); break;   \
+        case 8: e = launch_mc<R, NT, 8>(C, d, states, step_limit, nl_sys, nt, st); break;   \
+        default: e = launch_mc<R, NT, 16>(C, d, states, step_limit, nl_sys, nt, st); break; \
     }
     if (prec == ALMA_PREC_FP64) {
-        if (nt == 512) { ALMA_MC_CASE(double, 512) } else { ALMA_MC_CASE(double, 256) }
+        if (nt <= 512) { ALMA_MC_CASE(double, 512) } else { ALMA_MC_CASE(double, 1024) }
     } else {
-        if (nt == 512) { ALMA_MC_CASE(float, 512) } else { ALMA_MC_CASE(float, 256) }
+        if (nt <= 512) { ALMA_MC_CASE(float, 512) } else { ALMA_MC_CASE(float, 1024) }
     }
 #undef ALMA_MC_CASE
     if (e != cudaSuccess) return alma_cuda_error(e, "alma_mc_run launch");

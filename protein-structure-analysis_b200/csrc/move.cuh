@@ -103,7 +103,8 @@ struct CrossCand {
     double r2o, r2n;
     int j, gj;
 };
-constexpr int CROSS_BUF = 64;  // per warp: < 32 waiting + one batch of 32
+constexpr int CROSS_BUF = 64;  // per warp: < 32 waiting + one batch of 32 (also the
+                               // buffer of the SASA rows)
 constexpr int MAX_ROT = 2;
 constexpr int MAX_WPR = 4;  // segments (tasks) per moved-atom row, at most
 
@@ -141,14 +142,6 @@ struct MoveScratch {
 
 constexpr int QUEUE_PER_PARITY = 8;
 constexpr int QUEUE_PER_SYS = 2 * QUEUE_PER_PARITY;
-
-// Next task index of a dynamically scheduled phase for the calling warp
-// (lane 0 draws from the team's counter; every lane gets it).
-__device__ __forceinline__ int64_t draw_task(int *counter, int lane) {
-    int v = 0;
-    if (lane == 0) v = atomicAdd(counter, 1);
-    return __shfl_sync(0xffffffffu, v, 0);
-}
 
 // A j-side: sorted explicit atoms side_idx[eb, ee) plus the range [lo, hi).
 struct SideRef {
@@ -201,23 +194,34 @@ struct MoveDesc {
 };
 
 // Rodrigues rotation about unit axis u anchored at o (physics_engine.cpp:1848-1862).
+// Its operations are spelled out so that every kernel moves an atom to the
+// same bits.
+__device__ __forceinline__ double cross1(double a, double b, double c, double d) {  // a b - c d
+    return __fma_rn(a, b, -__dmul_rn(c, d));
+}
+
 __device__ __forceinline__ void rodrigues(double &px, double &py, double &pz, const Rot &R) {
-    const double vx = px - R.o[0], vy = py - R.o[1], vz = pz - R.o[2];
-    const double dot = R.u[0] * vx + R.u[1] * vy + R.u[2] * vz;
-    const double cx = R.u[1] * vz - R.u[2] * vy;
-    const double cy = R.u[2] * vx - R.u[0] * vz;
-    const double cz = R.u[0] * vy - R.u[1] * vx;
-    const double k = 1.0 - R.c;
-    px = R.o[0] + vx * R.c + cx * R.s + R.u[0] * dot * k;
-    py = R.o[1] + vy * R.c + cy * R.s + R.u[1] * dot * k;
-    pz = R.o[2] + vz * R.c + cz * R.s + R.u[2] * dot * k;
+    const double vx = __dsub_rn(px, R.o[0]), vy = __dsub_rn(py, R.o[1]), vz = __dsub_rn(pz, R.o[2]);
+    const double dot = __fma_rn(R.u[2], vz, __fma_rn(R.u[0], vx, __dmul_rn(R.u[1], vy)));
+    const double cx = cross1(R.u[1], vz, R.u[2], vy);
+    const double cy = cross1(R.u[2], vx, R.u[0], vz);
+    const double cz = cross1(R.u[0], vy, R.u[1], vx);
+    const double k = __dsub_rn(1.0, R.c);
+    px = __fma_rn(__dmul_rn(R.u[0], dot), k, __fma_rn(cx, R.s, __fma_rn(vx, R.c, R.o[0])));
+    py = __fma_rn(__dmul_rn(R.u[1], dot), k, __fma_rn(cy, R.s, __fma_rn(vy, R.c, R.o[1])));
+    pz = __fma_rn(__dmul_rn(R.u[2], dot), k, __fma_rn(cz, R.s, __fma_rn(vz, R.c, R.o[2])));
 }
 
 // Axis from atom ai to aj at the given positions; false when degenerate.
+// XFIRST: the order in which the squares of its length are added, kept as it
+// always was for a crankshaft's second axis, so that chains stay the same to
+// the last bit (the list's cell of the extreme atoms hangs on it).
+template <bool XFIRST = false>
 __device__ __forceinline__ bool make_axis(Rot &R, double4 pi, double4 pj, double delta) {
     R.o[0] = pi.x; R.o[1] = pi.y; R.o[2] = pi.z;
     double ux = pj.x - pi.x, uy = pj.y - pi.y, uz = pj.z - pi.z;
-    const double l = sqrt(ux * ux + uy * uy + uz * uz);
+    const double xy = XFIRST ? __fma_rn(uy, uy, __dmul_rn(ux, ux)) : __fma_rn(ux, ux, __dmul_rn(uy, uy));
+    const double l = sqrt(__fma_rn(uz, uz, xy));
     if (l < 1e-10) return false;
     ux /= l; uy /= l; uz /= l;
     R.u[0] = ux; R.u[1] = uy; R.u[2] = uz;
@@ -261,7 +265,7 @@ __device__ inline void decode_move(MoveDesc &M, const AlmaTopo &t, const double 
         if (side_has(R1.side, t.side_idx, bi)) rodrigues(pb4.x, pb4.y, pb4.z, R1);
         if (side_has(R1.side, t.side_idx, bj)) rodrigues(pj4.x, pj4.y, pj4.z, R1);
         Rot &R2 = M.rot[1];
-        if (!make_axis(R2, pb4, pj4, 0.0)) return;
+        if (!make_axis<true>(R2, pb4, pj4, 0.0)) return;
         R2.c = R1.c;   // cos(-d) = cos(d)
         R2.s = -R1.s;  // the reference passes (cosD, -sinD)
         R2.side = psi;
@@ -400,59 +404,141 @@ __device__ __forceinline__ double born_new_of(const MoveScratch &w, const double
     return 1.0 / fmax(1.0 / prm64[4 * (size_t)m + 1] - 0.5 * sum, 2.0);
 }
 
-// SASA change of affected atom k of system s: the ordered recurrence over
-// its half row (or short half row) at the new geometry, minus the old term
-// — read from b.sasa when the batch carries the current per-atom terms,
-// else recomputed at the old geometry in the same pass (the two
-// recurrences are independent and interleaved).  The new term goes to
-// dE_atom[2i] for the commit, the change to dE_atom[2i+1].  One warp.
-__device__ __forceinline__ void sasa_row(const MoveCtx &C, int s, int k, bool short_rows, double pi2, double pi4,
-                                         int lane, unsigned long long &nsasa) {
+// SASA change of up to four affected atoms of system s (4 k ... 4 k + 3 of the
+// list), eight lanes each: the ordered recurrence over the atom's half row (or
+// short half row) at the new geometry, minus the old term — read from b.sasa
+// when the batch carries the current per-atom terms, else recomputed at the
+// old geometry in the same pass.  The new term goes to dE_atom[2i] for the
+// commit, the change to dE_atom[2i+1].  A short row has 20-40 entries and its
+// recurrence is a chain of dependent FP64 steps: four chains side by side
+// share the warp's latency, where a row per warp had most of its lanes idle.
+// An entry out of reach takes 0 off, which changes nothing.
+__device__ __forceinline__ void sasa_rows(const MoveCtx &C, int s, int k4, int naff,
+                                          bool short_rows, int lane, unsigned long long &nsasa) {
     const AlmaBatch &b = C.b;
     const MoveScratch &w = C.w;
-    const int a0 = b.atom_off[s];
-    const int i = w.affected[a0 + k];
-    const bool moved = w.group[i] != 0;
+    const int sub = lane & ~7, sl = lane & 7;
+    const int k = 4 * k4 + (lane >> 3);
+    const bool valid = k < naff;
     const bool cached = b.sasa != nullptr;
-    const double4 pio = ld_xyz(b.xyz, i), pin = moved ? ld_xyz(w.xyz_new, i) : pio;
-    const double rsi = b.prm64[4 * (size_t)i + 1] + C.P.probe_r;
-    const double cs = pi2 * rsi * rsi;
-    double sao = pi4 * rsi * rsi, san = sao;
-    const uint32_t *rc = short_rows ? C.nl.shalf_cols : C.nl.half_cols;
-    const int64_t beg = short_rows ? C.nl.shalf_ptr[i] : C.nl.half_ptr[i];
-    const int64_t end = beg + (short_rows ? C.nl.shalf_len[i] : C.nl.half_len[i]);
-    uint32_t nxt = beg + lane < end ? rc[beg + lane] : 0u;
-    for (int64_t e0 = beg; e0 < end; e0 += 32) {
-        const int64_t e = e0 + lane;
-        double co = 0.0, cn = 0.0;
-        bool ho = false, hn = false;
-        if (e < end) {
-            const int j = (int)(nxt & ALMA_IDX_MASK);
-            if (e + 32 < end) nxt = rc[e + 32];  // next entry in flight
-            const double rsj = b.prm64[4 * (size_t)j + 1] + C.P.probe_r;
-            const double dc = rsi + rsj;
-            const double4 pjn = pos_new_eager(b.xyz, w.xyz_new, w.group, j);
-            const double4 pjo = ld_xyz(b.xyz, j);
-            if (!cached) {
-                const double ro = sqrt(d2_of(pio, pjo));
-                if (ro < dc) { ho = true; co = cs * ((dc - ro) / (2.0 * rsi)); }
-            }
-            const double rn = sqrt(d2_of(pin, pjn));
-            if (rn < dc) { hn = true; cn = cs * ((dc - rn) / (2.0 * rsi)); }
-        }
-        const unsigned mo = __ballot_sync(0xffffffffu, ho), mn = __ballot_sync(0xffffffffu, hn);
-        if (cached)  // independent recurrences, in row order (interleaved when both run)
-            san = sasa_chunk(san, mn, cn, lane);
-        else
-            sasa_chunk2(sao, mo, co, san, mn, cn, lane);
+    const int i = valid ? w.affected[b.atom_off[s] + k] : 0;
+    int64_t at = 0;
+    int len = 0;
+    double rsi = 1.0, told = 0.0;
+    double4 pio = make_double4(0.0, 0.0, 0.0, 0.0), pin = pio;
+    if (valid) {
+        at = short_rows ? C.nl.shalf_ptr[i] : C.nl.half_ptr[i];
+        len = short_rows ? C.nl.shalf_len[i] : C.nl.half_len[i];
+        rsi = b.prm64[4 * (size_t)i + 1] + C.P.probe_r;
+        pio = ld_xyz(b.xyz, i);
+        pin = pos_new_eager(b.xyz, w.xyz_new, w.group, i);
+        if (cached) told = b.sasa[i];
     }
-    if (lane == 0) {
+    const double cs = 2.0 * 3.14159265358979323846 * rsi * rsi;
+    double san = 4.0 * 3.14159265358979323846 * rsi * rsi, sao = san;
+    const int longest = __reduce_max_sync(0xffffffffu, len);
+    const uint32_t *rc = (short_rows ? C.nl.shalf_cols : C.nl.half_cols) + at;
+    uint32_t nxt = sl < len ? rc[sl] : 0u;
+    for (int e0 = 0; e0 < longest; e0 += 8) {
+        const int e = e0 + sl;
+        double co = 0.0, cn = 0.0;
+        if (e < len) {
+            const int j = (int)(nxt & ALMA_IDX_MASK);
+            if (e + 8 < len) nxt = rc[e + 8];  // next entry in flight
+            const double4 pjn = pos_new_eager(b.xyz, w.xyz_new, w.group, j);
+            const double dc = rsi + (b.prm64[4 * (size_t)j + 1] + C.P.probe_r);
+            const double rn = sqrt(d2_of(pin, pjn));
+            if (rn < dc) cn = cs * ((dc - rn) / (2.0 * rsi));
+            if (!cached) {
+                const double ro = sqrt(d2_of(pio, ld_xyz(b.xyz, j)));
+                if (ro < dc) co = cs * ((dc - ro) / (2.0 * rsi));
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) san = sasa_step(san, __shfl_sync(0xffffffffu, cn, sub + q));
+        if (!cached)
+#pragma unroll
+            for (int q = 0; q < 8; ++q) sao = sasa_step(sao, __shfl_sync(0xffffffffu, co, sub + q));
+    }
+    if (valid && sl == 0) {
         const double tn = C.P.gamma_sa * fmax(0.0, san);
-        const double to = cached ? b.sasa[i] : C.P.gamma_sa * fmax(0.0, sao);
+        const double to = cached ? told : C.P.gamma_sa * fmax(0.0, sao);
         w.dE_atom[2 * (size_t)i] = tn;
         w.dE_atom[2 * (size_t)i + 1] = tn - to;
+        nsasa += (cached ? 1ull : 2ull) * (unsigned long long)len;
     }
-    nsasa += (cached ? 1ull : 2ull) * (unsigned long long)(end - beg);
+}
+
+// SASA change of affected atom k of system s, one warp: entries within reach
+// (widened past the rounding of its square) wait in `buf` until 32 of them
+// share the FP64 square root and division, then take their steps in row order.
+struct SasaCand {
+    double r2, dc;
+};
+
+template <bool NEW>
+__device__ __forceinline__ double sasa_warp(const MoveCtx &C,
+                                            const uint32_t *rc, int len, double4 pi, double rsi, SasaCand *buf,
+                                            int lane) {
+    const AlmaBatch &b = C.b;
+    const double cs = 2.0 * 3.14159265358979323846 * rsi * rsi;
+    double sa = 4.0 * 3.14159265358979323846 * rsi * rsi;
+    auto steps = [&](int n) {
+        double cap = 0.0;
+        if (lane < n) {
+            const double r = sqrt(buf[lane].r2), dc = buf[lane].dc;
+            if (r < dc) cap = cs * ((dc - r) / (2.0 * rsi));
+        }
+        sa = sasa_steps(sa, n, cap);
+    };
+    int n = 0;
+    uint32_t nxt = lane < len ? rc[lane] : 0u;
+    for (int e0 = 0; e0 < len; e0 += 32) {
+        bool hit = false;
+        SasaCand c = {0.0, 0.0};
+        if (e0 + lane < len) {
+            const int j = (int)(nxt & ALMA_IDX_MASK);
+            if (e0 + 32 + lane < len) nxt = rc[e0 + 32 + lane];  // next entry in flight
+            c.dc = rsi + (b.prm64[4 * (size_t)j + 1] + C.P.probe_r);
+            c.r2 = d2_of(pi, NEW ? pos_new_eager(b.xyz, C.w.xyz_new, C.w.group, j) : ld_xyz(b.xyz, j));
+            hit = c.r2 < c.dc * c.dc * (1.0 + 1e-14);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (hit) buf[n + __popc(m & ((1u << lane) - 1u))] = c;
+        n += __popc(m);
+        __syncwarp();
+        if (n >= 32) {
+            steps(32);
+            n -= 32;
+            if (lane < n) c = buf[32 + lane];
+            __syncwarp();
+            if (lane < n) buf[lane] = c;
+            __syncwarp();
+        }
+    }
+    steps(n);
+    __syncwarp();
+    return sa;
+}
+
+__device__ __forceinline__ void sasa_row(const MoveCtx &C, int s, int k,
+                                         bool short_rows, SasaCand *buf, int lane, unsigned long long &nsasa) {
+    const AlmaBatch &b = C.b;
+    const MoveScratch &w = C.w;
+    const int i = w.affected[b.atom_off[s] + k];
+    const bool cached = b.sasa != nullptr;
+    const uint32_t *rc = short_rows ? C.nl.shalf_cols + C.nl.shalf_ptr[i] : C.nl.half_cols + C.nl.half_ptr[i];
+    const int len = short_rows ? C.nl.shalf_len[i] : C.nl.half_len[i];
+    const double rsi = b.prm64[4 * (size_t)i + 1] + C.P.probe_r;
+    const double4 pio = ld_xyz(b.xyz, i);
+    const double told = cached ? b.sasa[i] : C.P.gamma_sa * fmax(0.0, sasa_warp<false>(C, rc, len, pio, rsi, buf, lane));
+    const double4 pin = pos_new_eager(b.xyz, w.xyz_new, w.group, i);
+    const double tn = C.P.gamma_sa * fmax(0.0, sasa_warp<true>(C, rc, len, pin, rsi, buf, lane));
+    if (lane == 0) {
+        w.dE_atom[2 * (size_t)i] = tn;
+        w.dE_atom[2 * (size_t)i + 1] = tn - told;
+        nsasa += (cached ? 1ull : 2ull) * (unsigned long long)len;
+    }
 }
 
 // Whole-team evaluation of a decoded, non-degenerate proposal of system s.
@@ -555,12 +641,14 @@ __device__ MoveResult move_eval(const MoveCtx &C, const MoveDesc &M, int s, doub
     // segments so that there are about two tasks per warp.
     // Only edge members take part in cross pairs, so only their new radii
     // enter ΔE; the other members' radii are computed by the commit.
-    const int nw = T.gwarps();
+    // The first task of a warp is its own number, so the first draw is in
+    // flight while it runs; the counter counts the tasks past those.
+    const int nw = T.gwarps(), gw = T.gwarp();
     int wph = 1;
     while (wph < MAX_WPR && 2 * ne * wph < 2 * (int64_t)nw) wph *= 2;
     const int64_t nhct = ne * wph;
     int nx = 0;
-    for (int64_t it = draw_task(q + 4, lane); it < 2 * nhct; it = __shfl_sync(0xffffffffu, nx, 0)) {
+    for (int64_t it = gw; it < 2 * nhct; it = nw + (int64_t)__shfl_sync(0xffffffffu, nx, 0)) {
         if (lane == 0) nx = atomicAdd(q + 4, 1);  // the next draw, in flight during this task
         const bool marking = it >= nhct;
         const int64_t i2 = marking ? it - nhct : it;
@@ -570,8 +658,11 @@ __device__ MoveResult move_eval(const MoveCtx &C, const MoveDesc &M, int s, doub
         const int m = by_edge ? w.edge[a0 + k] : member(M, t.side_idx, k, g);
         const double4 pm = ld_xyz(w.xyz_new, m);
         if (!marking) {
-        R qm, rm, em;
-        prm_of<R>(b.prm, b.prm64, m, qm, rm, em);
+        auto radius = [&](int j) {
+            if constexpr (sizeof(R) == 4) return b.prm[4 * (size_t)j + 1];
+            else return b.prm64[4 * (size_t)j + 1];
+        };
+        const R rm = radius(m);
         double sum = 0.0;
         const int64_t hb = C.nl.half_ptr[m], he = hb + C.nl.half_len[m];
         // the next entry of the row is fetched while this one is evaluated
@@ -581,8 +672,7 @@ __device__ MoveResult move_eval(const MoveCtx &C, const MoveDesc &M, int s, doub
         for (; e < he; e += stp) {
             const int j = (int)(nxt & ALMA_IDX_MASK);
             if (e + stp < he) nxt = C.nl.half_cols[e + stp];
-            R qj, rj, ej;
-            prm_of<R>(b.prm, b.prm64, j, qj, rj, ej);
+            const R rj = radius(j);
             const double r2d = d2_of(pm, pos_new_eager(b.xyz, w.xyz_new, w.group, j));
             const R r2 = (R)r2d;
             sum += (double)hct_term<R>(f_sqrt(r2), r2, rm, rj);
@@ -627,28 +717,35 @@ __device__ MoveResult move_eval(const MoveCtx &C, const MoveDesc &M, int s, doub
         t0 = t1;
     }
 
-    // P3: cross pairs from the members' full rows (old and new geometry in
-    // one pass), then SASA of the affected atoms (old and new, in row
-    // order); boundary dihedrals and disulfides strided over threads.
-    // One task space: cross-pair segments first (every warp gets one when
-    // the rows allow), then the affected atoms' SASA, which wraps round onto
-    // the warps: a short SASA row after a half row beats a full row.
-    // Drawn from the team's counter like P2: the SASA rows first (each an
-    // ordered recurrence, the longest tasks), then the cross-pair segments.
+    // P3: SASA of the affected atoms and cross pairs from the edge members' full
+    // rows (old and new geometry in one pass); boundary dihedrals and disulfides
+    // strided over threads.  One task space, drawn from the team's counter like
+    // P2: the SASA rows first (each an ordered recurrence, the longest tasks),
+    // then the cross-pair segments.
     const int naff = q[3];
+    // Four SASA rows side by side when the warps have a dozen or more each; a
+    // row each when the phase is as long as its longest task.  256 chains of
+    // 50-600 residues, 50 proposals: 126 ms (always a row each 132, always
+    // four 134); one chain of 1.1k atoms, 16 CTAs and 4 teams: 26 us a proposal
+    // (26, 28); of 4.9k atoms: 60 (62, 67).
+    const bool four = naff >= 12 * nw;
+    const int nrow = four ? (naff + 3) >> 2 : naff;
     int wpc = 1;
-    while (wpc < MAX_WPR && ne * wpc + naff < 2 * (int64_t)nw) wpc *= 2;
+    while (wpc < MAX_WPR && ne * wpc + nrow < 2 * (int64_t)nw) wpc *= 2;
     const int64_t ncross = ne * wpc;
-    const double pi4 = 4.0 * 3.14159265358979323846, pi2 = 2.0 * 3.14159265358979323846;
     unsigned long long nsasa = 0;
-    for (int64_t it = draw_task(q + 0, lane); it < ncross + naff; it = __shfl_sync(0xffffffffu, nx, 0)) {
+    for (int64_t it = gw; it < ncross + nrow; it = nw + (int64_t)__shfl_sync(0xffffffffu, nx, 0)) {
         if (lane == 0) nx = atomicAdd(q + 0, 1);  // the next draw, in flight during this task
-        if (it < naff) {
-            sasa_row(C, s, (int)it, short_rows, pi2, pi4, lane, nsasa);
+        if (it < nrow) {
+            if (four)
+                sasa_rows(C, s, (int)it, naff, short_rows, lane, nsasa);
+            else
+                sasa_row(C, s, (int)it, short_rows,
+                         reinterpret_cast<SasaCand *>(cq + (threadIdx.x >> 5) * CROSS_BUF), lane, nsasa);
             continue;
         }
-        const int64_t k = (it - naff) / wpc;
-        const int seg = (int)((it - naff) % wpc);
+        const int64_t k = (it - nrow) / wpc;
+        const int seg = (int)((it - nrow) % wpc);
         int g;
         const int m = by_edge ? w.edge[a0 + k] : member(M, t.side_idx, k, g);
         const int gm = by_edge ? (int)w.group[m] : g + 1;
@@ -737,6 +834,8 @@ __device__ MoveResult move_eval(const MoveCtx &C, const MoveDesc &M, int s, doub
             atomicAdd(&w.ctr[4 * s + 0], (unsigned long long)npair);
         }
     }
+    nsasa += __shfl_xor_sync(0xffffffffu, nsasa, 8);  // the four rows of a task
+    nsasa += __shfl_xor_sync(0xffffffffu, nsasa, 16);
     if (lane == 0 && nsasa) atomicAdd(&w.ctr[4 * s + 2], nsasa);
     double ddih = 0.0, dss = 0.0;
     for (int r = t.dih_off[s] + tid; r < t.dih_off[s + 1]; r += nthr) {

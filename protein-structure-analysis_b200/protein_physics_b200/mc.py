@@ -70,8 +70,8 @@ def auto_shape(nsys, sms=None, sizes=None):
     proposal's time goes with the atoms and falls nearly in step with the
     cluster, so the cluster is then the smallest that takes the largest system
     below 0.4 of the work per SM: 256 chains of 50-600 residues,
-    50 proposals each, take 407 ms with one CTA of 512 threads, 228 with two,
-    171 with four, 179 with eight."""
+    50 proposals each, take 178 ms on clusters of two 1,024-thread CTAs, 126 on
+    four, 151 on eight."""
     if sms is None:
         sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
     cl = next((c for c in (16, 8, 4, 2) if nsys * c <= sms), 1)
@@ -174,7 +174,7 @@ class MCRunner:
             cfg = _lib.AlmaMCConfig.from_buffer_copy(self.cfg)
             self._tail_order = _t(order, torch.int32)  # alive until the state read after the launch
             cfg.sys_order, cfg.launch_systems = _ptr(self._tail_order), int(n)
-            cfg.cluster_size, cfg.spec_teams, cfg.threads_per_system = int(cl), int(k), 512
+            cfg.cluster_size, cfg.spec_teams, cfg.threads_per_system = int(cl), int(k), 0
             rc = self._run(cfg, step_limit)
             if rc == _lib.ALMA_EINVAL and k > 1 and b"resident" in self.L.alma_last_error():
                 cfg.spec_teams = 1
@@ -264,8 +264,9 @@ def autotune(batch, temperatures, seed, policy=0, moveset=None, proposals=200, c
         return _TUNED[key]
     if candidates is None:
         wide = max(2 * sms, 8 * batch.nsys if 2 * batch.nsys > sms else 0)  # queued systems: up to 8-CTA clusters
-        candidates = [(cl, nt, 1) for cl in (1, 2, 4, 8, 16) for nt in (256, 512) if batch.nsys * cl <= wide]
-        candidates += [(cl, 512, k) for cl in (8, 16) for k in (2, 4, 8) if batch.nsys * cl * k <= sms]
+        candidates = [(cl, nt, 1) for cl in (1, 2, 4, 8, 16) for nt in (0, 512) if batch.nsys * cl <= wide]
+        candidates += [(cl, nt, k) for cl in (8, 16) for nt in (0, 512) for k in (2, 4, 8)
+                       if batch.nsys * cl * k <= sms]
     xyz0, born0 = batch.xyz.clone(), batch.born.clone()
     best, best_rate = None, -1.0
     for cand in candidates:

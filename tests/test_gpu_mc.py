@@ -307,3 +307,28 @@ def test_second_runner_on_a_used_batch(cluster, before):
     x0, acc0, e0 = chain(fresh())
     assert acc == acc0 and e == e0
     np.testing.assert_array_equal(x, x0)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("cluster,teams", [(1, 1), (2, 1), (4, 1), (8, 1), (2, 3)])
+def test_threads_by_size_make_the_same_chain(cluster, teams, precision):
+    """The CTA size is a matter of speed alone: left to the size rule (1,024
+    threads where a system has 256 atoms per CTA or more, mixed precision) or
+    asked for, 256 and 512 threads, the chain keeps its decisions, and its
+    coordinates to the bit while they do (a moved atom's position does not
+    depend on who moves it); the energy differs by the order of its FP64 sums
+    (60 changes of terms below 1e5 kcal/mol: 60 x 1e5 x 2^-52 = 1e-9).  The
+    clusters take 657 atoms to both sides of the rule, and the SASA rows to
+    both sides of theirs (a dozen a warp, of 8 warps to 64)."""
+    from protein_physics_b200.device import DeviceBatch
+    from protein_physics_b200.mc import MCRunner
+    g, F = _setup("insulin")
+    out = []
+    for threads in (0, 256, 512):
+        b = DeviceBatch([(g["xyz"], g["q"], g["r"], g["eps"], F)], precision=precision)
+        st = MCRunner(b, 0.6, 21, cluster_size=cluster, threads=threads, spec_teams=teams).run_to(60)
+        out.append((b.coords(0), int(st["n_accepted"][0]), int(st["n_rebuild"][0]), float(st["energy"][0])))
+    for x, acc, reb, e in out[1:]:
+        assert (acc, reb) == out[0][1:3]
+        np.testing.assert_array_equal(x, out[0][0])
+        assert e == pytest.approx(out[0][3], rel=1e-10, abs=1e-8)
