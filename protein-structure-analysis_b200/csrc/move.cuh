@@ -212,16 +212,14 @@ __device__ __forceinline__ void rodrigues(double &px, double &py, double &pz, co
     pz = __fma_rn(__dmul_rn(R.u[2], dot), k, __fma_rn(cz, R.s, __fma_rn(vz, R.c, R.o[2])));
 }
 
-// Axis from atom ai to aj at the given positions; false when degenerate.
-// XFIRST: the order in which the squares of its length are added, kept as it
-// always was for a crankshaft's second axis, so that chains stay the same to
-// the last bit (the list's cell of the extreme atoms hangs on it).
-template <bool XFIRST = false>
+// Axis from atom ai to aj at the given positions; false when degenerate.  The
+// order of the squares in its length is spelled out like the rotation: a chain
+// stays the same to the last bit (the list's cell of the extreme atoms hangs
+// on it).
 __device__ __forceinline__ bool make_axis(Rot &R, double4 pi, double4 pj, double delta) {
     R.o[0] = pi.x; R.o[1] = pi.y; R.o[2] = pi.z;
     double ux = pj.x - pi.x, uy = pj.y - pi.y, uz = pj.z - pi.z;
-    const double xy = XFIRST ? __fma_rn(uy, uy, __dmul_rn(ux, ux)) : __fma_rn(ux, ux, __dmul_rn(uy, uy));
-    const double l = sqrt(__fma_rn(uz, uz, xy));
+    const double l = sqrt(__fma_rn(uz, uz, __fma_rn(ux, ux, __dmul_rn(uy, uy))));
     if (l < 1e-10) return false;
     ux /= l; uy /= l; uz /= l;
     R.u[0] = ux; R.u[1] = uy; R.u[2] = uz;
@@ -265,7 +263,7 @@ __device__ inline void decode_move(MoveDesc &M, const AlmaTopo &t, const double 
         if (side_has(R1.side, t.side_idx, bi)) rodrigues(pb4.x, pb4.y, pb4.z, R1);
         if (side_has(R1.side, t.side_idx, bj)) rodrigues(pj4.x, pj4.y, pj4.z, R1);
         Rot &R2 = M.rot[1];
-        if (!make_axis<true>(R2, pb4, pj4, 0.0)) return;
+        if (!make_axis(R2, pb4, pj4, 0.0)) return;
         R2.c = R1.c;   // cos(-d) = cos(d)
         R2.s = -R1.s;  // the reference passes (cosD, -sinD)
         R2.side = psi;
