@@ -264,13 +264,13 @@ __device__ __forceinline__ V6 block_scan6(V6 x, V6 *sm, V6 &total) {
 }
 
 // Torsion gradient.  A bond's sum runs over an atom range [lo, hi) plus a few
-// explicit atoms; as prefixes within tiles of TG_TILE atoms and tile totals it
-// is prefix(hi) - prefix(lo) + the totals of the tiles between, which a warp
-// adds with one tile per lane.  Two launches over all tiles and all bonds
-// instead of one CTA per system that scans and then walks its bonds (16k
-// atoms, 4,000 bonds, one system: 372 -> 10 us), and no long prefix whose
-// difference cancels.
-constexpr int TG_TILE = 256;
+// explicit atoms; the range is prefix(hi) - prefix(lo), a prefix the sum of the
+// tiles before the atom, tile after tile, plus its place in its own tile: the
+// order in which one CTA scans a system.  The order is kept for the sake of the
+// sampler, whose chains follow the last bit of the gradient (an extreme atom
+// sits on a cell face of the list); tiles and bonds of all systems run at once
+// instead (16k atoms, 4,000 bonds, one system: 372 -> 13 us in two launches).
+constexpr int TG_TILE = 1024;
 
 __device__ __forceinline__ V6 torque_of(const double *xyz, const double *grad, int m, double4 c) {
     const double4 p = ld_xyz(xyz, m), g = ld_xyz(grad, m);
@@ -321,19 +321,34 @@ torsion_grad_kernel(const int32_t *__restrict__ atom_off, int nsys, const double
     V6 S = {};
     for (int64_t e = t.side_ptr[k] + lane; e < t.side_ptr[k + 1]; e += 32)
         S = v6_add(S, torque_of(xyz, grad, t.side_idx[e], c));
-    const int lo = t.side_lo[k] - a0, hi = t.side_hi[k] - a0;  // within the system
-    if (hi > lo) {
-        const int base = tile_base<TG_TILE>(atom_off, s), tl = lo / TG_TILE, th = (hi - 1) / TG_TILE;
-        for (int q = tl + lane; q < th; q += 32)
-            for (int d = 0; d < 6; ++d) S.v[d] += tot[6 * (size_t)(base + q) + d];
-    }
     for (int q = 0; q < 6; ++q) S.v[q] = warp_sum(S.v[q]);
-    if (lane == 0) {
-        if (hi > lo) {
-            const double *ph = P + 6 * (size_t)(a0 + hi - 1), *pl = P + 6 * (size_t)(a0 + lo - 1);
-            const bool first = lo % TG_TILE == 0;  // the range starts a tile: nothing before it to take off
-            for (int q = 0; q < 6; ++q) S.v[q] += ph[q] - (first ? 0.0 : pl[q]);
+    const int lo = t.side_lo[k], hi = t.side_hi[k];
+    if (hi > lo) {
+        // lane q < 6: component q of the range
+        const int a1 = atom_off[s + 1], q = lane < 6 ? lane : 0;
+        const double *ts = tot + 6 * (size_t)tile_base<TG_TILE>(atom_off, s) + q;
+        const int tl = (lo - a0) / TG_TILE, th = hi < a1 ? (hi - a0) / TG_TILE : (a1 - a0 - 1) / TG_TILE + 1;
+        double carry = 0.0, before = 0.0;
+#pragma unroll 8
+        for (int u = 0; u < th; ++u) {
+            if (u == tl) before = carry;
+            carry += ts[6 * (size_t)u];
         }
+        if (th == tl) before = carry;
+        auto pick = [&](const V6 &x) {
+            double r = x.v[0];
+#pragma unroll
+            for (int d = 1; d < 6; ++d) r = q == d ? x.v[d] : r;
+            return r;
+        };
+        double ph = carry;
+        if (hi < a1) ph = carry + P[6 * (size_t)hi + q] - pick(torque_of(xyz, grad, hi, c));
+        const double pl = before + P[6 * (size_t)lo + q] - pick(torque_of(xyz, grad, lo, c));
+        const double sum = pick(S) + (ph - pl);
+#pragma unroll
+        for (int d = 0; d < 6; ++d) S.v[d] = __shfl_sync(0xffffffffu, sum, d);
+    }
+    if (lane == 0) {
         const double4 pi = ld_xyz(xyz, t.rb_ij[2 * k]), pj = ld_xyz(xyz, t.rb_ij[2 * k + 1]);
         double ux = pj.x - pi.x, uy = pj.y - pi.y, uz = pj.z - pi.z;
         const double l = sqrt(ux * ux + uy * uy + uz * uz);
