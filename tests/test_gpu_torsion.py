@@ -267,7 +267,7 @@ def test_mala_graph_replay_equals_eager():
         assert np.array_equal(out[0][0][k], out[1][0][k]), k
 
 
-@pytest.mark.parametrize("residues", [(16, 5, 31), (170,), (300,), (620,)])
+@pytest.mark.parametrize("residues", [(16, 5, 31), (62, 63, 64, 65), (170,), (300,), (620,)])
 def test_torsion_tiles_and_clusters(residues):
     """Chains whose atoms end inside, at and past a tile of the prefix sums,
     and whose bond counts take each cluster size: the torsion gradient of a
