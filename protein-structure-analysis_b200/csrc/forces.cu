@@ -6,12 +6,13 @@
 //
 //   pair   warp per atom over its FULL row: the direct pair force of every
 //          non-excluded partner within 12 Å, gathered (each pair is seen
-//          from both ends, so no atomics), and dE/da_i = Σ_j ∂e/∂(a_i a_j)·a_j;
-//          zeroes the atom's fixed-point slots;
+//          from both ends, so no atomics), and dE/da_i = Σ_j ∂e/∂(a_i a_j)·a_j,
+//          left as the coefficient c_i of the Born pass; zeroes the atom's
+//          fixed-point slots;
 //   sasa   warp per atom over its HALF row: the SASA recurrence
-//          sa <- sa - min(0.85 sa, cap_k) (:2068-2083) is run twice — once to
-//          count the entries that took the 0.85·sa branch, once to give each
-//          entry that took the cap branch its adjoint γ·π·R*·0.15^(number of
+//          sa <- sa - min(0.85 sa, cap_k) (:2068-2083) over the entries within
+//          reach counts those that took the 0.85·sa branch; each entry that
+//          took the cap branch then gets its adjoint γ·π·R*·0.15^(number of
 //          later 0.85 entries); the pair force goes to both atoms through
 //          64-bit fixed-point atomics (integer adds: order independent);
 //   bonded thread per dihedral record / disulfide, fixed-point atomics.  The
