@@ -265,8 +265,10 @@ def _kernel_roofline(runner, batch, tuned, proposals_per_launch, workload=None):
     d = c1 - c0
     ops = d[0] * OPS_PAIR + d[1] * OPS_HCT + d[2] * OPS_SASA
     achieved = ops / (k_ms * 1e-3)
-    name = ("mc_spec_kernel<float,%d,%d> x %d teams" % (tuned[1], tuned[0], tuned[2]) if tuned[2] > 1 else
-            "mc_kernel<float,%d,%d>" % (tuned[1] or 512, tuned[0]))
+    # CTA size 0: chosen by the library from the atoms per CTA
+    threads = tuned[1] or (1024 if batch.natoms >= 256 * tuned[0] * batch.nsys else 512)
+    name = ("mc_spec_kernel<float,%d,%d> x %d teams" % (threads, tuned[0], tuned[2]) if tuned[2] > 1 else
+            "mc_kernel<float,%d,%d>" % (threads, tuned[0]))
     nprop = float(np.sum(st1["step"] - st0["step"]))
     per = DRAM_BYTES_PER_PROPOSAL.get(workload)
     traffic = per * nprop if per else None
