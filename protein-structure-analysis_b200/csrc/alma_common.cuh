@@ -248,11 +248,10 @@ __device__ __forceinline__ double pair_delta(const DevParams &P, double r2o, dou
         const float kap = (float)P.kappa;
         const float gdo = (float)P.coulomb_over_epsw * qp * rio * __expf(-kap * ro);
         const float ddh = gdo * expm1f(-kap * dr - log1pf(dr * rio));
-        float xo = 0.0f, xn = 0.0f;  // below the last bit of f² for far pairs (GB_FAR)
-        if (ro2 < GB_FAR * aao || rn2 < GB_FAR * aan) {
-            xo = aao * __expf(-0.25f * __fdividef(ro2, aao));
-            xn = aan * __expf(-0.25f * __fdividef(rn2, aan));
-        }
+        // also where they are below the last bit of f² (GB_FAR): num compares
+        // their difference with d2, which may be smaller still
+        const float xo = aao * __expf(-0.25f * __fdividef(ro2, aao));
+        const float xn = aan * __expf(-0.25f * __fdividef(rn2, aan));
         const float fo2 = ro2 + xo, fn2 = rn2 + xn;
         const float fo = fo2 * rsqrtf(fo2), fn = fn2 * rsqrtf(fn2);
         const float num = (float)(-d2) + (xo - xn);

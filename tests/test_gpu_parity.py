@@ -361,3 +361,53 @@ def test_nl_rows_at_the_edges(oracle, kind):
         keep = fcols > J  # the full row holds the half row in its order
         assert np.array_equal(fcols[keep], ocols), s
         assert need[s, 0] == len(fcols) and need[s, 1] == len(ocols)
+
+
+def _one_bond_system(xyz, q, r, eps, side):
+    """A system of loose atoms and one rotatable bond 1-2 whose j-side is the
+    atom range `side`."""
+    import dataclasses
+    from protein_physics_b200.device import _empty_topo
+    flat = dataclasses.replace(
+        _empty_topo(len(q)), rb_i=np.array([1], np.int32), rb_j=np.array([2], np.int32),
+        rb_kind=np.array([2], np.int32), rb_scale=np.ones(1), side_ptr=np.zeros(2, np.int64),
+        side_lo=np.array([side[0]], np.int32), side_hi=np.array([side[1]], np.int32),
+        side_count=np.array([side[1] - side[0]], np.int64))
+    return np.asarray(xyz, np.float64), np.asarray(q, np.float64), np.asarray(r, np.float64), \
+        np.asarray(eps, np.float64), flat
+
+
+def test_move_gb_change_of_far_pairs(oracle):
+    """A pair whose distance stays while a Born radius changes: its GB energy
+    changes by C qq (fo² - fn²) / (fo fn (fo + fn)), and fo² - fn² lies all in
+    the exponentials A exp(-r²/4A), however far below the last bit of f² these
+    are.  Atom 2 turns about its own axis: it stays where it is and takes its
+    half-list radius, without the descreening by atoms 0 and 1; r² is 61-70
+    times the larger A = a_0 a_2.  Tolerance: the argument r²/4A <= 17.5 is good
+    to 4 x 2^-23 and the exponential to 22 x 2^-23 on top, 1.1e-5 of each term;
+    the terms differ by a factor of 10 or more, the other factors are good to
+    1e-6."""
+    from protein_physics_b200.device import DeviceBatch
+    r = np.array([0.42, 1.2, 0.35])
+    systems = []
+    for m in (61.0, 63.5, 66.0, 70.0):
+        x = np.array([[3.0, 0.0, 0.0], [0.0, 0.0, 1.3], [0.0, 0.0, 0.0]])
+        for _ in range(50):  # the radii depend a little on the distance
+            a = oracle.born_radii(x, r, oracle.nl_build(x))
+            x[0, 0] = np.sqrt(m * a[0] * a[2])
+        systems.append(_one_bond_system(x, [1.0, 0.0, 1.0], r, np.zeros(3), (2, 3)))
+    b = DeviceBatch(systems)
+    b.build_nl()
+    b.born_radii()
+    a = b.born.cpu().numpy().reshape(-1, 3)
+    d2 = np.array([s[0][0, 0] ** 2 for s in systems])
+    Ao, An = a[:, 0] * a[:, 2], a[:, 0] * r[2]  # no atom follows atom 2: its half row is empty
+    xo, xn = Ao * np.exp(-d2 / (4 * Ao)), An * np.exp(-d2 / (4 * An))
+    assert np.all(a[:, 2] < 0.5) and np.all(xo > 10 * xn)
+    assert np.all(d2 > 60.5 * Ao) and np.all(d2 < 70.5 * Ao)
+    fo, fn = np.sqrt(d2 + xo), np.sqrt(d2 + xn)
+    p = b.params
+    gb = -0.5 * (1.0 / p.eps_prot - 1.0 / p.eps_water) * p.coulomb
+    k = np.zeros(len(systems), int)
+    _, terms = b.move_dE(k, k, np.full((len(systems), 2), 0.4))
+    np.testing.assert_allclose(terms[:, 0].cpu().numpy(), gb * (xo - xn) / (fo * fn * (fo + fn)), rtol=1.5e-5)
