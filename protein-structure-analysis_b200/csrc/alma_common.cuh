@@ -111,14 +111,6 @@ __device__ __forceinline__ double m_abs(double x) { return fabs(x); }
 __device__ __forceinline__ float f_sqrt(float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; }
 __device__ __forceinline__ double f_sqrt(double x) { return sqrt(x); }
 
-// 1/x in FP64 from an FP32 estimate y0 of it (within a few 2^-22) and one
-// Newton step, y1 = y0 (2 - x y0): relative error below 2^-40.  For quotients
-// that are rounded to FP32 next, or multiply an FP32 factor.
-__device__ __forceinline__ double recip_from(double x, float y0) {
-    const double y = (double)y0;
-    return fma(y, fma(-x, y, 1.0), y);
-}
-
 // LJ + hard core of a contact inside sigma (r2d < sig2), FP64: the steep
 // terms, where a clash's r^-12 would amplify the FP32 rounding of sigma
 // twelvefold.
@@ -213,14 +205,14 @@ __device__ __forceinline__ double m_log1p(double x) { return log1p(x); }
 // LJ 12-6 + capped hard core of one pair (r2 in FP64).  Inside sigma the
 // terms grow steeply and are evaluated in FP64 with FP64 sigma and
 // epsilon (sig64 = R*_i + R*_j, eps64 = eps_i eps_j); outside, in
-// precision R (FP32: s² from an FP64 quotient, rinv = 1/r).
+// precision R from the FP64 quotient s².
 template <typename R>
 __device__ __forceinline__ double lj_hard(const DevParams &P, double r2, R sig, R eps_prod, double sig64,
-                                          double eps64, R rinv) {
+                                          double eps64) {
     const double sig2 = sig64 * sig64;
     if (r2 < sig2) return lj_contact(P, r2, sig2, sig64, eps64);
     if constexpr (sizeof(R) == 4) {
-        const float s2 = (float)__dmul_rn(sig2, recip_from(r2, __fmul_rn(rinv, rinv)));
+        const float s2 = (float)(sig2 / r2);
         const float s6 = __fmul_rn(__fmul_rn(s2, s2), s2);
         return (double)__fmul_rn(__fmul_rn(4.0f, sqrtf(eps_prod)), __fmaf_rn(s6, s6, -s6));
     }
@@ -257,7 +249,7 @@ __device__ __forceinline__ double pair_delta(const DevParams &P, double r2o, dou
         const float num = (float)(-d2) + (xo - xn);
         const float dgb = (float)P.gb_coef * qp * __fdividef(num, fo * fn * (fo + fn));
         return (double)ddh + (double)dgb +
-               (lj_hard<float>(P, r2n, sig, eps_prod, sig64, eps64, rin) - lj_hard<float>(P, r2o, sig, eps_prod, sig64, eps64, rio));
+               (lj_hard<float>(P, r2n, sig, eps_prod, sig64, eps64) - lj_hard<float>(P, r2o, sig, eps_prod, sig64, eps64));
     }
     const double d2 = r2n - r2o;
     const R ro2 = (R)r2o, rn2 = (R)r2n;
@@ -271,7 +263,7 @@ __device__ __forceinline__ double pair_delta(const DevParams &P, double r2o, dou
     const R num = (R)(-d2) + (xo - xn);
     const R dgb = (R)P.gb_coef * qp * num / (fo * fn * (fo + fn));
     return (double)ddh + (double)dgb +
-           (lj_hard<R>(P, r2n, sig, eps_prod, sig64, eps64, (R)0) - lj_hard<R>(P, r2o, sig, eps_prod, sig64, eps64, (R)0));
+           (lj_hard<R>(P, r2n, sig, eps_prod, sig64, eps64) - lj_hard<R>(P, r2o, sig, eps_prod, sig64, eps64));
 }
 
 // HCT descreening integral of atom j (radius rj) on atom i (radius ri).

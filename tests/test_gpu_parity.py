@@ -411,3 +411,42 @@ def test_move_gb_change_of_far_pairs(oracle):
     k = np.zeros(len(systems), int)
     _, terms = b.move_dE(k, k, np.full((len(systems), 2), 0.4))
     np.testing.assert_allclose(terms[:, 0].cpu().numpy(), gb * (xo - xn) / (fo * fn * (fo + fn)), rtol=1.5e-5)
+
+
+def test_move_lj_outside_sigma_is_rounded_once():
+    """LJ of a pair just outside sigma, where s² = sigma²/r² is an FP64
+    quotient rounded to FP32: the quotients lie 1-4 FP64 ulps above the middle
+    of two FP32 values, so that an approximate one falls to the other side.
+    There 4 (s¹² - s⁶) changes by 12 for s², and an ulp of it (2^-24) is worth
+    7e-7.  The moved atom goes to 11.5 Å, where the term is below 0.02 kcal/mol
+    and its FP32 roundings are below 5 x 2^-24 of it, 6e-9."""
+    from fractions import Fraction
+    from protein_physics_b200.device import DeviceBatch
+    rng = np.random.default_rng(3)
+    f32 = np.float32
+    systems, old = [], []
+    while len(systems) < 64:
+        r = float(rng.integers(3 << 20, 9 << 19)) / (1 << 20)  # r² exact
+        lo = f32(rng.uniform(0.99993, 0.99998))
+        mid = (float(lo) + float(np.nextafter(lo, f32(1)))) / 2
+        sig = np.sqrt(mid * r * r)
+        for _ in range(16):
+            if sig * sig / (r * r) > mid:
+                break
+            sig = np.nextafter(sig, 10.0)
+        s2 = sig * sig / (r * r)
+        if not mid < s2 <= mid * (1 + 2.0 ** -50):
+            continue
+        u = f32(s2)
+        s6 = f32(f32(u * u) * u)
+        old.append(4.0 * float(f32(float(Fraction(float(s6)) ** 2 - Fraction(float(s6))))))
+        cx = (r + 11.5) / 2  # half a turn about the axis through (cx, 0): r -> 11.5
+        x = [[0.0, 0.0, 0.0], [cx, 0.0, -5.0], [cx, 0.0, -6.5], [r, 0.0, 0.0]]
+        systems.append(_one_bond_system(x, np.zeros(4), [1.0, 0.01, 0.01, sig - 1.0], [1.0, 0.0, 0.0, 1.0], (3, 4)))
+    b = DeviceBatch(systems)
+    b.build_nl()
+    b.born_radii()
+    k = np.zeros(len(systems), int)
+    _, terms = b.move_dE(k, k, np.full((len(systems), 2), np.pi))
+    s6 = np.array([(s[2].sum() - 0.02) / 11.5 for s in systems]) ** 6
+    np.testing.assert_allclose(terms[:, 0].cpu().numpy(), 4 * (s6 * s6 - s6) - np.array(old), rtol=0, atol=2e-8)
