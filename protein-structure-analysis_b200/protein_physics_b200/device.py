@@ -286,12 +286,34 @@ class DeviceBatch:
     def _sp(self):
         return C.c_void_p((self.stream or torch.cuda.current_stream()).cuda_stream)
 
+    def _cells_needed(self):
+        """Cells of all systems' grids at the current coordinates (the grid of
+        alma_nl_build: cells of 14 Å + 1e-6, one more on every side of the box)."""
+        cs = float(np.sqrt(196.0)) + 1e-6
+        x = self.xyz[:self.natoms, :3].cpu().numpy()
+        total = 0
+        for s in range(self.nsys):
+            xs = x[self.atom_off_h[s]:self.atom_off_h[s + 1]]
+            if len(xs):
+                lo, hi = xs.min(0), xs.max(0)
+                cells = float(np.prod(np.maximum(1.0, np.ceil((hi - (lo - cs) + 2.0 * cs) / cs))))
+                if not cells < 2.0 ** 31:  # the list's cell index is 32-bit
+                    raise RuntimeError(f"neighbor list: system {s} spans {(hi - lo).max():.3g} Å, its grid has "
+                                       f"{cells:.3g} cells")
+                total += int(cells)
+        return total
+
     def build_nl(self, sys_mask=None, check=True):
-        """Neighbor lists (all systems, or those with sys_mask[s] != 0)."""
+        """Neighbor lists (all systems, or those with sys_mask[s] != 0).  With
+        check, grids and rows that do not fit are given the space they need and
+        the list is built again; a list that cannot be built raises."""
         if self.natoms == 0:
             self.nl_ready = True
             return
-        for attempt in range(3):
+        # the need of cells is known from the coordinates, that of rows from a
+        # build whose cells fit: rows, cells, rows is the longest way (a masked
+        # build first, then all systems)
+        for attempt in range(4):
             b, t, nl = self.batch_s, self.topo_s, self.nl_s
             rc = self.L.alma_nl_build(C.byref(b), C.byref(t) if self.use_topo else None, C.byref(nl),
                                       C.byref(self.params), _ptr(sys_mask) if sys_mask is not None else None,
@@ -301,22 +323,22 @@ class DeviceBatch:
             if not check:
                 break
             st = int(self.status.item())
-            if st & (_lib.ST_NL_OVERFLOW | _lib.ST_CELL_OVERFLOW):
-                need = self.need.cpu().numpy()
-                self.status.zero_()
-                if st & _lib.ST_CELL_OVERFLOW:  # a system whose grid did not fit has no row counts yet
-                    self.max_cells *= 4
-                    self.nl_ws = torch.zeros(self.L.alma_nl_workspace_bytes(self.nsys, self.natoms, self.max_cells),
-                                             dtype=torch.uint8, device=_DEV)
-                else:
-                    keep_cells = self.max_cells
-                    self._alloc_nl(need)
-                    self.max_cells = keep_cells
-                    self.nl_ws = torch.zeros(self.L.alma_nl_workspace_bytes(self.nsys, self.natoms, self.max_cells),
-                                             dtype=torch.uint8, device=_DEV)
-                sys_mask = None
-                continue
-            break
+            if not st & (_lib.ST_NL_OVERFLOW | _lib.ST_CELL_OVERFLOW):
+                break
+            self.nl_ready = False
+            self.status.zero_()
+            sys_mask = None
+            if st & _lib.ST_CELL_OVERFLOW:  # a system whose grid did not fit has no row counts yet
+                cells = self._cells_needed()
+                self.max_cells = max(self.max_cells, cells + cells // 4)
+            else:
+                keep_cells = self.max_cells
+                self._alloc_nl(self.need.cpu().numpy())
+                self.max_cells = keep_cells
+            self.nl_ws = torch.zeros(self.L.alma_nl_workspace_bytes(self.nsys, self.natoms, self.max_cells),
+                                     dtype=torch.uint8, device=_DEV)
+        else:
+            raise RuntimeError("neighbor list: overflow persists")
         self.nl_ready = True
 
     def compact_nl(self):

@@ -450,3 +450,54 @@ def test_move_lj_outside_sigma_is_rounded_once():
     _, terms = b.move_dE(k, k, np.full((len(systems), 2), np.pi))
     s6 = np.array([(s[2].sum() - 0.02) / 11.5 for s in systems]) ** 6
     np.testing.assert_allclose(terms[:, 0].cpu().numpy(), 4 * (s6 * s6 - s6) - np.array(old), rtol=0, atol=2e-8)
+
+
+def _spread_system(extent, seed, n=24):
+    """Atoms in two clumps at opposite corners of a box of `extent` Å."""
+    rng = np.random.default_rng(seed)
+    x = rng.uniform(0, 12, (n, 3))
+    x[n // 2:] += extent
+    return x, rng.choice([-0.4, 0.4], n), np.full(n, 1.7), np.full(n, 0.1), None
+
+
+@pytest.mark.parametrize("rows", ["roomy", "tight"])
+def test_nl_of_atoms_far_apart(oracle, rows):
+    """Systems whose grids hold many times the cells that were allotted, alone
+    or together with rows that do not fit: cells and rows are regrown in turn
+    until the list is complete."""
+    from protein_physics_b200.device import DeviceBatch
+
+    class Tight(DeviceBatch):
+        NL_FULL_PER_ATOM = 1
+        NL_HALF_PER_ATOM = 1
+        NL_SHORT_PER_ATOM = 2
+
+    # rows far past the tight regions (one entry per atom and 64 more)
+    rng = np.random.default_rng(4)
+    dense = (rng.uniform(0, 30, (1400, 3)), np.zeros(1400), np.full(1400, 1.7), np.full(1400, 0.1), None)
+    systems = [_spread_system(1000.0, 1), dense, _spread_system(40.0, 2), _spread_system(700.0, 3)]
+    b = (Tight if rows == "tight" else DeviceBatch)(systems, precision="fp64")
+    cells = [np.prod(np.ceil((np.ptp(s[0], axis=0) + 3 * 14.000001) / 14.000001)) for s in systems]
+    assert sum(cells) > 16 * b.max_cells
+    terms = b.energy_terms().cpu().numpy()
+    for s, (x, q, r, e, _) in enumerate(systems):
+        rp, cols, _ = b.nl_host(s, half=True)
+        ptr, ocols = oracle.nl_build(x)
+        assert np.array_equal(rp, ptr) and np.array_equal(cols, ocols), s
+        assert terms[s, 4] == pytest.approx(oracle.calculate_potential(x, q, r, e)[4], rel=1e-10)
+
+
+def test_nl_that_cannot_be_built_raises():
+    """A box with more cells than the list can index is an error, not a list
+    without pairs; the batch works again with coordinates that fit."""
+    from protein_physics_b200.device import DeviceBatch
+    x, q, r, e, _ = _spread_system(1.0e6, 5)
+    b = DeviceBatch([(x, q, r, e, None)])
+    with pytest.raises(RuntimeError, match="neighbor list"):
+        b.energy_terms()
+    with pytest.raises(RuntimeError, match="neighbor list"):
+        b.evaluate()
+    near = _spread_system(5.0, 5)
+    b.load_coords(near[0])
+    want = DeviceBatch([near]).energy_terms()
+    assert torch.equal(b.energy_terms(), want)
