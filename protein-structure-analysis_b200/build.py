@@ -56,13 +56,14 @@ def build(force=False, verbose=False):
         # an object is rebuilt when its source or any header is newer than it
         if not force and os.path.exists(obj) and os.path.getmtime(obj) > max(os.path.getmtime(src), newest_header):
             continue
-        cmd = [NVCC, *ARCH, *FLAGS, "-I" + INCLUDE, "-I" + CSRC, "-c", src, "-o", obj]
-        if verbose:
-            cmd.insert(1, "-Xptxas=-v")
+        # registers and spills of every kernel, kept beside the object
+        cmd = [NVCC, "-Xptxas=-v", *ARCH, *FLAGS, "-I" + INCLUDE, "-I" + CSRC, "-c", src, "-o", obj]
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT)))
     failed = []
     for src, p in procs:
         out, _ = p.communicate()
+        with open(os.path.join(objdir, os.path.basename(src) + ".ptxas"), "wb") as f:
+            f.write(out)
         if verbose or p.returncode != 0:
             sys.stdout.write(out.decode(errors="replace"))
         if p.returncode != 0:

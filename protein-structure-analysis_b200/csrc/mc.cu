@@ -349,9 +349,14 @@ __device__ bool team_rebuild(const MoveCtx &C, const MCConfigDev &cfg, int s, co
 // cluster keeps its own copy of the chain state and makes the same draws
 // and decisions (the ΔE totals are bit-identical in every CTA); rank 0
 // writes the state back.
+//
+// One CTA per SM is all the launches ask for, and said so in the bounds: 512
+// threads then get up to 128 registers, where the compiler by itself stops at
+// 64 and spills 0.6-1.1 KB (40 FP64 chains of 300 residues on 2-CTA clusters:
+// 2,340 us a proposal at 64 registers, 1,942 here).
 template <typename R, int NT, int CL>
-__global__ void __launch_bounds__(NT) mc_kernel(MoveCtx C, MCConfigDev cfg,
-                                                          AlmaChainState *__restrict__ states, int64_t step_limit) {
+__global__ void __launch_bounds__(NT, 1) mc_kernel(MoveCtx C, MCConfigDev cfg,
+                                                   AlmaChainState *__restrict__ states, int64_t step_limit) {
     __shared__ MoveDesc M;
     __shared__ double sm[128];
     __shared__ double part[8];
@@ -578,7 +583,7 @@ __global__ void spec_wait_selftest_kernel(SpecRound *Rd, uint32_t *status, int32
 }
 
 template <typename R, int NT, int CL>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, 1)
 mc_spec_kernel(MoveCtx C, MCConfigDev cfg, AlmaChainState *__restrict__ states, int64_t step_limit, int teams,
                size_t team_stride, SpecRound *__restrict__ rounds) {
     __shared__ MoveDesc M;
