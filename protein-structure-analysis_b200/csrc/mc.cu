@@ -841,11 +841,14 @@ extern "C" int alma_mc_run(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *
     // per SM.  Threads per CTA: the caller's choice, or by size.  1,024 at 64
     // registers hide the latency of the row scans better than 512 at 128, in
     // spite of some spilled registers, where an average system has an atom for
-    // every four threads or more (256 chains of 50-600 residues on 4-CTA
-    // clusters: 126 ms for 50 proposals against 159; one chain of 4.9k atoms,
-    // 16 CTAs and 4 teams: 60 us a proposal against 63); with less the barriers
-    // of twice the warps cost more than that (1.1k atoms on 16 CTAs: 28 against
-    // 26).  FP64 pair terms need the registers.
+    // every four threads or more; with less the barriers of twice the warps cost
+    // more than that.  One team, 512 / 1,024 threads, us a proposal, 4 chains:
+    // 64 residues on 1, 4, 8, 16 CTAs (1,089 to 68 atoms each) 352 / 281,
+    // 147 / 137, 112 / 115, 100 / 115; 300 residues on 4, 16 CTAs 380 / 304,
+    // 161 / 156.  256 chains of 50-600 residues on 4-CTA clusters, 50
+    // proposals: 169 / 132 ms.  256 threads are slower everywhere (600 chains of
+    // 30 residues: 1,096 / 746 / 638 us).  Four teams of 16 CTAs: 63 / 60 us
+    // for 4.9k atoms, 26 / 28 for 1.1k.  FP64 pair terms need the registers.
     int nt = cfg->threads_per_system;
     if (nt != 0 && nt != 256 && nt != 512)
         return alma_set_error(ALMA_EINVAL, "alma_mc_run: threads_per_system must be 0, 256 or 512");
@@ -869,7 +872,7 @@ extern "C" int alma_mc_run(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *
         default: e = launch_mc_spec<R, NT, 16>(C, d, states, step_limit, nl_sys, nt, teams, stride, rounds, st, &fits); break; \
     }
         if (prec == ALMA_PREC_FP64) {
-            if (nt <= 512) { ALMA_SPEC_CASE(double, 512) } else { ALMA_SPEC_CASE(double, 1024) }
+            ALMA_SPEC_CASE(double, 512)
         } else {
             if (nt <= 512) { ALMA_SPEC_CASE(float, 512) } else { ALMA_SPEC_CASE(float, 1024) }
         }
@@ -895,7 +898,7 @@ extern "C" int alma_mc_run(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *
         default: e = launch_mc<R, NT, 16>(C, d, states, step_limit, nl_sys, nt, st); break; \
     }
     if (prec == ALMA_PREC_FP64) {
-        if (nt <= 512) { ALMA_MC_CASE(double, 512) } else { ALMA_MC_CASE(double, 1024) }
+        ALMA_MC_CASE(double, 512)
     } else {
         if (nt <= 512) { ALMA_MC_CASE(float, 512) } else { ALMA_MC_CASE(float, 1024) }
     }
