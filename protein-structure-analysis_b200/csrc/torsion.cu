@@ -195,28 +195,67 @@ __device__ __forceinline__ void apply_torsions(const Bonds &B, int (*any_of)[8],
     sync();  // no CTA leaves while another may still read its shared memory
 }
 
+struct ApplyArgs {
+    const int32_t *atom_off;
+    double *xyz;
+    AlmaTopo t;
+    const int32_t *rb_parent, *atom_rb;
+    const double *delta;
+    const uint8_t *mask;
+    double *Tbuf;
+    int32_t *Pbuf;
+};
+
 template <int CL>
-__global__ void __launch_bounds__(COMPOSE_THREADS)
-torsion_apply_kernel(const int32_t *__restrict__ atom_off, double *xyz, AlmaTopo t,
-                     const int32_t *__restrict__ rb_parent, const int32_t *__restrict__ atom_rb,
-                     const double *__restrict__ delta, const uint8_t *__restrict__ mask, int nrb_total, double *Tbuf,
-                     int32_t *Pbuf) {
+__device__ __forceinline__ void apply_system(const ApplyArgs &A, int s) {
     extern __shared__ double compose_smem[];
     __shared__ int any_of[2][8];  // per round parity and CTA of the cluster: bonds still climbing
     const int rank = CL > 1 ? (int)cg::this_cluster().block_rank() : 0;
-    const int s = blockIdx.x / CL;
-    if (mask && !mask[s]) return;  // the whole cluster
-    const int r0 = t.rb_off[s], nr = t.rb_off[s + 1] - r0;
+    const int r0 = A.t.rb_off[s], nr = A.t.rb_off[s + 1] - r0;
     const int per = max(1, (nr + CL - 1) / CL);
     const int k0 = min(nr, rank * per), k1 = min(nr, k0 + per);
-    const int a0 = atom_off[s], a1 = atom_off[s + 1];
+    const int a0 = A.atom_off[s], a1 = A.atom_off[s + 1];
     if (per <= COMPOSE_HOLD) {
         const SharedBonds<CL> B{compose_smem, reinterpret_cast<int32_t *>(compose_smem + 24 * COMPOSE_HOLD), per};
-        apply_torsions<CL>(B, any_of, rank, k0, k1, r0, a0, a1, xyz, t, rb_parent, atom_rb, delta);
+        apply_torsions<CL>(B, any_of, rank, k0, k1, r0, a0, a1, A.xyz, A.t, A.rb_parent, A.atom_rb, A.delta);
     } else {
-        const GlobalBonds B{{Tbuf + 12 * (size_t)r0, Tbuf + 12 * ((size_t)nrb_total + r0)},
-                            {Pbuf + r0, Pbuf + nrb_total + r0}};
-        apply_torsions<CL>(B, any_of, rank, k0, k1, r0, a0, a1, xyz, t, rb_parent, atom_rb, delta);
+        const size_t n = (size_t)A.t.nrb;
+        const GlobalBonds B{{A.Tbuf + 12 * (size_t)r0, A.Tbuf + 12 * (n + r0)}, {A.Pbuf + r0, A.Pbuf + n + r0}};
+        apply_torsions<CL>(B, any_of, rank, k0, k1, r0, a0, a1, A.xyz, A.t, A.rb_parent, A.atom_rb, A.delta);
+    }
+}
+
+template <int CL>
+__global__ void __launch_bounds__(COMPOSE_THREADS) torsion_apply_kernel(ApplyArgs A, int limit) {
+    const int s = blockIdx.x / CL;
+    if (A.mask && !A.mask[s]) return;                          // the whole cluster
+    if (A.t.rb_off[s + 1] - A.t.rb_off[s] > limit) return;  // likewise
+    apply_system<CL>(A, s);
+}
+
+// An uneven batch: the host knows the number of systems and of bonds, not the
+// sizes, and shapes the clusters for the mean.  Systems of more bonds than
+// such a cluster holds (`limit`) are left to this kernel, a few clusters of 8 CTAs
+// that find them 512 systems at a time and share them out in order.  A batch
+// without any pays 2 us.  4,030 residues among 99 chains of 64: 2,761 us on
+// the one CTA of the mean (2,132 as one CTA of twice the threads, atoms apart),
+// 415 here; 1,000 among 40 of 64: 618 and 49.
+constexpr int LARGE_CTAS = 8, LARGE_CLUSTERS = 18;  // about a CTA per SM
+
+__global__ void __launch_bounds__(COMPOSE_THREADS) torsion_apply_large_kernel(ApplyArgs A, int nsys, int limit) {
+    __shared__ unsigned found[COMPOSE_THREADS / 32];
+    const int cluster = blockIdx.x / LARGE_CTAS, clusters = gridDim.x / LARGE_CTAS;
+    int seen = 0;
+    for (int s0 = 0; s0 < nsys; s0 += COMPOSE_THREADS) {
+        const int s = s0 + (int)threadIdx.x;
+        const bool large = s < nsys && (!A.mask || A.mask[s]) && A.t.rb_off[s + 1] - A.t.rb_off[s] > limit;
+        const unsigned m = __ballot_sync(0xffffffffu, large);
+        if ((threadIdx.x & 31) == 0) found[threadIdx.x >> 5] = m;
+        if (!__syncthreads_or(large)) continue;
+        for (int w = 0; w < COMPOSE_THREADS / 32; ++w)
+            for (unsigned rest = found[w]; rest; rest &= rest - 1u)
+                if (seen++ % clusters == cluster) apply_system<LARGE_CTAS>(A, s0 + 32 * w + __ffs(rest) - 1);
+        __syncthreads();  // found[] is written again
     }
 }
 
@@ -537,17 +576,25 @@ extern "C" int alma_torsion_apply(const AlmaBatch *b, const AlmaTopo *t, const A
     cudaStream_t st = (cudaStream_t)stream;
     double *Tbuf = (double *)workspace;
     int32_t *Pbuf = (int32_t *)((char *)workspace + align256(sizeof(double) * 24 * (size_t)t->nrb));
-    // About one bond per thread, up to 8 CTAs (the portable cluster): past
-    // that a wider cluster only adds barrier time.
+    // About one bond per thread of the mean system, up to 8 CTAs (the portable
+    // cluster): past that a wider cluster only adds barrier time.
     const int avg = t->nrb / b->nsys;
     const int cl = avg <= COMPOSE_THREADS ? 1 : avg <= 2 * COMPOSE_THREADS ? 2 : avg <= 4 * COMPOSE_THREADS ? 4 : 8;
-    auto kfn = cl == 1 ? torsion_apply_kernel<1> : cl == 2 ? torsion_apply_kernel<2>
-               : cl == 4 ? torsion_apply_kernel<4> : torsion_apply_kernel<8>;
-    ALMA_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COMPOSE_SMEM));
-    ALMA_CUDA_TRY(alma_launch_cluster(kfn, (unsigned)(b->nsys * cl), COMPOSE_THREADS, (unsigned)cl, COMPOSE_SMEM, st,
-                                      b->atom_off, b->xyz, *t, tree->rb_parent, tree->atom_rb, delta, sys_mask,
-                                      t->nrb, Tbuf, Pbuf));
-    ALMA_LAUNCH_CHECK("alma_torsion_apply");
+    const ApplyArgs A{b->atom_off, b->xyz, *t, tree->rb_parent, tree->atom_rb, delta, sys_mask, Tbuf, Pbuf};
+    auto launch = [&](auto kfn, int grid, int ctas, auto... args) {
+        const cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COMPOSE_SMEM);
+        if (e != cudaSuccess) return e;
+        return alma_launch_cluster(kfn, (unsigned)grid, COMPOSE_THREADS, (unsigned)ctas, COMPOSE_SMEM, st, A, args...);
+    };
+    const int limit = cl * COMPOSE_HOLD;
+    const bool large = b->nsys > 1 && cl < LARGE_CTAS && t->nrb > limit;  // there may be one
+    ALMA_CUDA_TRY(launch(cl == 1 ? torsion_apply_kernel<1> : cl == 2 ? torsion_apply_kernel<2>
+                         : cl == 4 ? torsion_apply_kernel<4> : torsion_apply_kernel<8>,
+                         b->nsys * cl, cl, large ? limit : 0x7fffffff));
+    if (large)
+        ALMA_CUDA_TRY(launch(torsion_apply_large_kernel, std::min(b->nsys, LARGE_CLUSTERS) * LARGE_CTAS, LARGE_CTAS,
+                             b->nsys, limit));
+    ALMA_LAUNCH_CHECK_N("alma_torsion_apply", large ? 2 : 1);
     return ALMA_OK;
 }
 

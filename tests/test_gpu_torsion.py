@@ -301,3 +301,59 @@ def test_torsion_tiles_and_clusters(residues):
         # sums of up to n torques of size |x| |g|, in FP64
         assert np.abs(gth[k0:k1] - ref).max() <= 1e-13 * flat.n * 100.0 * 10.0
         assert np.abs(b.coords(s) - _sequential(x, topos[s], flat, delta[k0:k1])).max() < 1e-9
+
+
+def _run_of_residues(name, residues, r0=0):
+    """(system, topology) of a run of residues of a benchmark chain."""
+    from conftest import ROOT
+    from protein_physics_b200.topology import BondTopology, flatten
+    w = np.load(os.path.join(ROOT, "workloads", name + ".npz"), allow_pickle=False)
+    ridx = w["res_idx"]
+    a, b = np.searchsorted(ridx, [r0, r0 + residues])
+    T = BondTopology()
+    T.build([str(v) for v in w["resnames"][a:b]], [str(v) for v in w["atomnames"][a:b]],
+            [int(v) - r0 for v in ridx[a:b]])
+    return (w["xyz"][a:b].astype(np.float64), w["charge"][a:b], w["radius"][a:b], w["epsilon"][a:b], flatten(T)), T
+
+
+def test_torsion_apply_of_uneven_batches():
+    """A chain of far more bonds than the mean (1,000 and more past what a CTA
+    of the batch's launch holds) is turned by a launch of its own: to the bit as
+    alone, first or last in the batch, masked or not."""
+    from protein_physics_b200.device import DeviceBatch
+    from protein_physics_b200.torsion import TorsionSpace
+    long, _ = _run_of_residues("c4_globule_1000res", 500)
+    short = [_run_of_residues("c4_globule_1000res", 6 + k % 5, 7 * k)[0] for k in range(40)]
+    rng = np.random.default_rng(2)
+    delta = [rng.normal(0, 0.05, s[4].nrb) for s in [long] + short]
+    alone = []
+    for s, d in zip([long] + short, delta):
+        b = DeviceBatch([s])
+        TorsionSpace(b).apply(torch.as_tensor(d, device="cuda"))
+        alone.append(b.coords(0))
+    for order in (list(range(41)), list(range(40, -1, -1))):
+        systems = [([long] + short)[k] for k in order]
+        assert sum(s[4].nrb for s in systems) / 41 < 512 < 1024 < long[4].nrb
+        for mask in (None, torch.tensor([k % 2 for k in order], dtype=torch.uint8, device="cuda")):
+            b = DeviceBatch(systems)
+            before = [b.coords(p) for p in range(41)]
+            TorsionSpace(b).apply(torch.as_tensor(np.concatenate([delta[k] for k in order]), device="cuda"),
+                                  sys_mask=mask)
+            for p, k in enumerate(order):
+                assert np.array_equal(b.coords(p), alone[k] if mask is None or k % 2 else before[p]), (p, k)
+
+
+def test_torsion_apply_past_the_shared_memory():
+    """A chain of more bonds than a cluster's shared memory holds (8 x 1,024)
+    takes the global buffers: 40 of its bonds turned, against numpy."""
+    from protein_physics_b200.device import DeviceBatch
+    from protein_physics_b200.torsion import TorsionSpace
+    system, T = _run_of_residues("c5_multidomain_4x1000res", 4030)
+    flat = system[4]
+    assert flat.nrb > 8 * 1024
+    rng = np.random.default_rng(6)
+    delta = np.zeros(flat.nrb)
+    delta[rng.choice(flat.nrb, 40, replace=False)] = rng.normal(0, 0.05, 40)
+    b = DeviceBatch([system])
+    TorsionSpace(b).apply(torch.as_tensor(delta, device="cuda"))
+    assert np.abs(b.coords(0) - _sequential(system[0], T, flat, delta)).max() < 1e-9
