@@ -237,9 +237,9 @@ __global__ void __launch_bounds__(COMPOSE_THREADS) torsion_apply_kernel(ApplyArg
 // sizes, and shapes the clusters for the mean.  Systems of more bonds than
 // such a cluster holds (`limit`) are left to this kernel, a few clusters of 8 CTAs
 // that find them 512 systems at a time and share them out in order.  A batch
-// without any pays 2 us.  4,030 residues among 99 chains of 64: 2,761 us on
+// without any pays 4-5 us.  4,030 residues among 99 chains of 64: 2,761 us on
 // the one CTA of the mean (2,132 as one CTA of twice the threads, atoms apart),
-// 415 here; 1,000 among 40 of 64: 618 and 49.
+// 435 here; 1,000 among 40 of 64: 618 and 50.
 constexpr int LARGE_CTAS = 8, LARGE_CLUSTERS = 18;  // about a CTA per SM
 
 __global__ void __launch_bounds__(COMPOSE_THREADS) torsion_apply_large_kernel(ApplyArgs A, int nsys, int limit) {
@@ -345,22 +345,43 @@ torsion_prefix_kernel(const int32_t *__restrict__ atom_off, int nsys, const doub
         for (int q = 0; q < 6; ++q) tot[6 * (size_t)blockIdx.x + q] = total.v[q];
 }
 
-// Warp per bond: the torsion derivative from the prefixes.
+// Eight lanes per bond: the torsion derivative from the prefixes.  A bond has
+// few explicit atoms and a serial tail (a root, three quotients), so a warp per
+// bond left most lanes idle and batches of many chains queued for it (400
+// chains of 64 residues, 102k bonds: 87 -> 37 us).  The explicit atoms are summed
+// as a warp would: atom e in the share of lane e mod 32, the shares by halves.
+constexpr int TG_LANES = 8;
+
 __global__ void __launch_bounds__(256)
 torsion_grad_kernel(const int32_t *__restrict__ atom_off, int nsys, const double *__restrict__ xyz,
                     const double *__restrict__ grad, AlmaTopo t, const uint8_t *__restrict__ mask,
                     const double *__restrict__ P, const double *__restrict__ tot, double *__restrict__ gtheta) {
-    const int k = blockIdx.x * 8 + ((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) / TG_LANES), lane = threadIdx.x % TG_LANES;
+    const unsigned group = 0xffu << (threadIdx.x & 24u);  // the lanes of this bond
     if (k >= t.nrb) return;
     const int s = sys_of_atom(t.rb_off, nsys, k);
     if (mask && !mask[s]) return;
     const int a0 = atom_off[s];
     if (atom_off[s + 1] <= a0) return;
     const double4 c = ld_xyz(xyz, a0);
-    V6 S = {};
-    for (int64_t e = t.side_ptr[k] + lane; e < t.side_ptr[k + 1]; e += 32)
-        S = v6_add(S, torque_of(xyz, grad, t.side_idx[e], c));
-    for (int q = 0; q < 6; ++q) S.v[q] = warp_sum(S.v[q]);
+    const int64_t e0 = t.side_ptr[k], e1 = t.side_ptr[k + 1];
+    auto share = [&](int u) {
+        V6 x = {};
+        for (int64_t e = e0 + TG_LANES * u + lane; e < e1; e += 32) x = v6_add(x, torque_of(xyz, grad, t.side_idx[e], c));
+        return x;
+    };
+    V6 S = share(0);
+    if (e1 - e0 > TG_LANES) {
+        S = v6_add(S, share(2));
+        V6 x = share(1);
+        x = v6_add(x, share(3));
+        S = v6_add(S, x);
+    }
+    __syncwarp(group);
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+#pragma unroll
+        for (int o = TG_LANES / 2; o > 0; o >>= 1) S.v[q] += __shfl_xor_sync(group, S.v[q], o);
     const int lo = t.side_lo[k], hi = t.side_hi[k];
     if (hi > lo) {
         // lane q < 6: component q of the range
@@ -385,7 +406,7 @@ torsion_grad_kernel(const int32_t *__restrict__ atom_off, int nsys, const double
         const double pl = before + P[6 * (size_t)lo + q] - pick(torque_of(xyz, grad, lo, c));
         const double sum = pick(S) + (ph - pl);
 #pragma unroll
-        for (int d = 0; d < 6; ++d) S.v[d] = __shfl_sync(0xffffffffu, sum, d);
+        for (int d = 0; d < 6; ++d) S.v[d] = __shfl_sync(group, sum, d, TG_LANES);
     }
     if (lane == 0) {
         const double4 pi = ld_xyz(xyz, t.rb_ij[2 * k]), pj = ld_xyz(xyz, t.rb_ij[2 * k + 1]);
@@ -560,8 +581,9 @@ extern "C" int alma_torsion_grad(const AlmaBatch *b, const AlmaTopo *t, const do
     double *tot = (double *)((char *)workspace + align256(sizeof(double) * 6 * (size_t)b->natoms));
     torsion_prefix_kernel<<<tile_slots<TG_TILE>(b->natoms, b->nsys), TG_TILE, 0, st>>>(b->atom_off, b->nsys, b->xyz,
                                                                                       grad, sys_mask, P, tot);
-    torsion_grad_kernel<<<(t->nrb + 7) / 8, 256, 0, st>>>(b->atom_off, b->nsys, b->xyz, grad, *t, sys_mask, P, tot,
-                                                          gtheta);
+    const int per_block = 256 / TG_LANES;
+    torsion_grad_kernel<<<(t->nrb + per_block - 1) / per_block, 256, 0, st>>>(b->atom_off, b->nsys, b->xyz, grad, *t,
+                                                                              sys_mask, P, tot, gtheta);
     ALMA_LAUNCH_CHECK_N("alma_torsion_grad", 2);
     return ALMA_OK;
 }

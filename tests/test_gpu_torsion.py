@@ -357,3 +357,45 @@ def test_torsion_apply_past_the_shared_memory():
     b = DeviceBatch([system])
     TorsionSpace(b).apply(torch.as_tensor(delta, device="cuda"))
     assert np.abs(b.coords(0) - _sequential(system[0], T, flat, delta)).max() < 1e-9
+
+
+def test_torsion_grad_of_any_side_list():
+    """Sides given as atom lists of every length class (none, one share of eight
+    lanes, several, more than a warp), with and without a range, in two systems
+    whose bond counts fill no block: against numpy.  Sums of up to n torques
+    |x| |g|, in FP64."""
+    import ctypes as C
+    import dataclasses
+    from protein_physics_b200 import _lib
+    from protein_physics_b200.device import DeviceBatch, _empty_topo, _ptr
+    rng = np.random.default_rng(12)
+    systems, sides = [], []
+    for n, nrb in ((130, 37), (90, 5)):
+        explicit = [np.sort(rng.choice(n, min(n, k), replace=False)).astype(np.int32)
+                    for k in ([0, 1, 7, 8, 9, 16, 17, 24, 31, 32, 33, 64, 70] * 3)[:nrb]]
+        lo = np.where(np.arange(nrb) % 3 == 0, 0, rng.integers(0, n // 2, nrb))
+        hi = np.where(np.arange(nrb) % 3 == 0, 0, rng.integers(n // 2, n + 1, nrb))
+        ij = np.stack([rng.choice(n, 2, replace=False) for _ in range(nrb)])
+        flat = dataclasses.replace(
+            _empty_topo(n), rb_i=ij[:, 0].astype(np.int32), rb_j=ij[:, 1].astype(np.int32),
+            rb_kind=np.zeros(nrb, np.int32), rb_scale=np.ones(nrb),
+            side_ptr=np.concatenate([[0], np.cumsum([len(e) for e in explicit])]).astype(np.int64),
+            side_idx=np.concatenate(explicit), side_lo=lo.astype(np.int32), side_hi=hi.astype(np.int32),
+            side_count=np.array([len(e) + h - l for e, l, h in zip(explicit, lo, hi)], np.int64))
+        systems.append((rng.uniform(0, 30, (n, 3)), np.zeros(n), np.full(n, 1.5), np.zeros(n), flat))
+        sides.append([np.concatenate([e, np.arange(l, h)]).astype(int) for e, l, h in zip(explicit, lo, hi)])
+    b = DeviceBatch(systems)
+    grad = np.zeros((b.natoms, 4))
+    grad[:, :3] = rng.normal(0, 10.0, (b.natoms, 3))
+    nrb = int(b.rb_off_h[-1])
+    ws = torch.zeros(b.L.alma_torsion_workspace_bytes(b.natoms, b.nsys, nrb), dtype=torch.uint8, device="cuda")
+    g, out = torch.as_tensor(grad, device="cuda"), torch.zeros(nrb, dtype=torch.float64, device="cuda")
+    _lib.check(b.L.alma_torsion_grad(C.byref(b.batch_s), C.byref(b.topo_s), _ptr(g), None, _ptr(ws), _ptr(out),
+                                     b._sp()), "alma_torsion_grad")
+    out = out.cpu().numpy()
+    for s, (x, _, _, _, flat) in enumerate(systems):
+        gs = grad[b.atom_off_h[s]:b.atom_off_h[s + 1], :3]
+        for k in range(flat.nrb):
+            u = x[flat.rb_j[k]] - x[flat.rb_i[k]]
+            ref = np.sum(np.cross(u / np.linalg.norm(u), x[sides[s][k]] - x[flat.rb_i[k]]) * gs[sides[s][k]])
+            assert abs(out[b.rb_off_h[s] + k] - ref) <= 1e-13 * 2 * flat.n * 52.0 * 40.0, (s, k)
