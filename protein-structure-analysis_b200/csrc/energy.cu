@@ -12,7 +12,7 @@
 //            recurrence sa -= min(0.85 sa, cap) is applied lane by lane),
 //            and evaluates pair_e (:2148-2164) for non-excluded entries with
 //            r² <= 12² (:2223-2232).
-//   reduce : one cluster per system — pair and SASA sums in a fixed order,
+//   reduce : one cluster or CTA per system — pair and SASA sums in a fixed order,
 //            plus the dihedral (:1912-1921) and disulfide (:1965-1974) terms.
 #include <cooperative_groups.h>
 
@@ -56,55 +56,67 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 4) pair_sasa_kernel(
                             buf[threadIdx.x >> 5], atom_e, sasa_out);
 }
 
-// One cluster of 8 CTAs per system: the atoms' and records' terms strided over
-// the cluster, CTA partials summed in rank order through distributed shared
-// memory.  The dihedral records are the work (an FP64 atan2 and a cosine per
-// term): one CTA took 52 us at 16k atoms and 234 us at 65k, the cluster
-// 8.5 and 28 us.  Always 8 CTAs, so that a chain's sums are the same
-// alone and in a batch.
-constexpr int REDUCE_CTAS = 8;
+// The atoms' and records' terms of a system in eight strided shares, each
+// summed by 256 threads, the shares' sums in order.  The dihedral records are
+// the work (an FP64 atan2 and a cosine per term).  One system: a cluster of 8
+// CTAs takes a share each and adds up through distributed shared memory (16k
+// atoms: 52 -> 8.5 us, 65k: 234 -> 28).  Many small systems: a CTA each, which
+// takes the shares one after the other.  The sums are the same either way, so
+// a chain's terms do not depend on the batch.
+constexpr int REDUCE_SHARES = 8;
 constexpr int REDUCE_THREADS = 256;
 
+template <int CTAS>
 __global__ void __launch_bounds__(REDUCE_THREADS)
 energy_reduce_kernel(DevParams P, const int32_t *__restrict__ atom_off, const double *__restrict__ xyz,
                      const double *__restrict__ atom_e, AlmaTopo t, int has_topo, const uint8_t *__restrict__ mask,
                      double *__restrict__ terms) {
-    __shared__ double sm[4][REDUCE_THREADS / 32], part[4];
-    cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank(), s = blockIdx.x / REDUCE_CTAS;
+    constexpr int PER = REDUCE_SHARES / CTAS, NW = REDUCE_THREADS / 32;  // shares per CTA
+    __shared__ double sm[PER][4][NW], part[PER][4];
+    const int rank = CTAS > 1 ? (int)cg::this_cluster().block_rank() : 0, s = blockIdx.x / CTAS;
     if (mask && !mask[s]) return;  // the whole cluster
-    const int tid = rank * REDUCE_THREADS + (int)threadIdx.x, nthr = REDUCE_CTAS * REDUCE_THREADS;
+    constexpr int stride = REDUCE_SHARES * REDUCE_THREADS;
     const int a0 = atom_off[s], a1 = atom_off[s + 1];
-    double v[4] = {0.0, 0.0, 0.0, 0.0};  // pairs, SASA, dihedrals, disulfides
-    for (int i = a0 + tid; i < a1; i += nthr) {
-        v[0] += atom_e[2 * (size_t)i];
-        v[1] += atom_e[2 * (size_t)i + 1];
-    }
-    if (has_topo) {
-        for (int r = t.dih_off[s] + tid; r < t.dih_off[s + 1]; r += nthr) v[2] += dih_record_energy(xyz, t, r);
-        for (int k = t.ss_off[s] + tid; k < t.ss_off[s + 1]; k += nthr) {
+    const int d0 = has_topo ? t.dih_off[s] : 0, d1 = has_topo ? t.dih_off[s + 1] : 0;
+    const int s0 = has_topo ? t.ss_off[s] : 0, s1 = has_topo ? t.ss_off[s + 1] : 0;
+    // shares past the longest list are empty: their sums are 0
+    const int longest = max(a1 - a0, max(d1 - d0, s1 - s0));
+    const int used = PER > 1 ? min(PER, (longest + REDUCE_THREADS - 1) / REDUCE_THREADS) : 1;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int u = 0; u < used; ++u) {
+        const int tid = (rank * PER + u) * REDUCE_THREADS + (int)threadIdx.x;
+        double v[4] = {0.0, 0.0, 0.0, 0.0};  // pairs, SASA, dihedrals, disulfides
+        for (int i = a0 + tid; i < a1; i += stride) {
+            v[0] += atom_e[2 * (size_t)i];
+            v[1] += atom_e[2 * (size_t)i + 1];
+        }
+        for (int r = d0 + tid; r < d1; r += stride) v[2] += dih_record_energy(xyz, t, r);
+        for (int k = s0 + tid; k < s1; k += stride) {
             const double dr = sqrt(dist2(xyz, t.ss_ij[2 * k], t.ss_ij[2 * k + 1])) - P.r0_ss;
             v[3] += P.k_ss * dr * dr;
         }
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        v[k] = warp_sum(v[k]);
-        if (lane == 0) sm[k][wid] = v[k];
+        for (int k = 0; k < 4; ++k) {
+            v[k] = warp_sum(v[k]);
+            if (lane == 0) sm[u][k][wid] = v[k];
+        }
     }
     __syncthreads();
-    if (threadIdx.x < 4) {
+    if (threadIdx.x < 4 * used) {
+        const int u = (int)threadIdx.x >> 2, k = threadIdx.x & 3;
         double q = 0.0;
-        for (int w = 0; w < REDUCE_THREADS / 32; ++w) q += sm[threadIdx.x][w];
-        part[threadIdx.x] = q;
+        for (int w = 0; w < NW; ++w) q += sm[u][k][w];
+        part[u][k] = q;
     }
-    cl.sync();
+    if constexpr (CTAS > 1) cg::this_cluster().sync();
+    else __syncthreads();
     if (rank == 0 && threadIdx.x == 0) {
-        double e[4];
+        double e[4] = {0.0, 0.0, 0.0, 0.0};
         for (int k = 0; k < 4; ++k) {
-            e[k] = 0.0;
-            for (int r = 0; r < REDUCE_CTAS; ++r) e[k] += cl.map_shared_rank(part, r)[k];
+            if constexpr (CTAS > 1)
+                for (int r = 0; r < CTAS; ++r) e[k] += cg::this_cluster().map_shared_rank(&part[0][0], r)[k];
+            else
+                for (int u = 0; u < used; ++u) e[k] += part[u][k];
         }
         const double sasa = (a1 > a0) ? P.beta_sa + e[1] : 0.0;
         double *o = terms + 5 * (size_t)s;
@@ -114,7 +126,7 @@ energy_reduce_kernel(DevParams P, const int32_t *__restrict__ atom_off, const do
         o[3] = e[0];
         o[4] = sasa + e[2] + e[3] + e[0];
     }
-    cl.sync();  // no CTA leaves before its partials are read
+    if constexpr (CTAS > 1) cg::this_cluster().sync();  // no CTA leaves before its partials are read
 }
 
 }  // namespace alma
@@ -164,9 +176,18 @@ extern "C" int alma_energy(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *
     AlmaTopo tt;
     if (t) tt = *t;
     else memset(&tt, 0, sizeof(tt));
-    ALMA_CUDA_TRY(alma_launch_cluster(energy_reduce_kernel, (unsigned)b->nsys * REDUCE_CTAS, REDUCE_THREADS,
-                                      REDUCE_CTAS, (size_t)0, st, P, b->atom_off, b->xyz, atom_e, tt, t != nullptr,
-                                      sys_mask, terms));
+    // A CTA per system where its serial shares are shorter than the queue of
+    // clusters: mean atoms up to 16 per system of the batch (64 x 1,089 atoms: 9.0 us
+    // either way; 300 x 2.4k: 20.7 against 29.9, 400 x 1,089: 12 and 36, 2,000 x
+    // 324: 21 and 137; 100 x 2.4k: 19.2 against 12.5, 128 x 4.9k: 26 and 18).
+    const bool one = (int64_t)b->natoms <= 16 * (int64_t)b->nsys * b->nsys;
+    if (one)
+        energy_reduce_kernel<1><<<b->nsys, REDUCE_THREADS, 0, st>>>(P, b->atom_off, b->xyz, atom_e, tt, t != nullptr,
+                                                                    sys_mask, terms);
+    else
+        ALMA_CUDA_TRY(alma_launch_cluster(energy_reduce_kernel<REDUCE_SHARES>, (unsigned)b->nsys * REDUCE_SHARES,
+                                          REDUCE_THREADS, REDUCE_SHARES, (size_t)0, st, P, b->atom_off, b->xyz, atom_e,
+                                          tt, t != nullptr, sys_mask, terms));
     ALMA_LAUNCH_CHECK_N("alma_energy", b->natoms > 0 ? 2 : 1);
     return ALMA_OK;
 }

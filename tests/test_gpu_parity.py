@@ -501,3 +501,24 @@ def test_nl_that_cannot_be_built_raises():
     b.load_coords(near[0])
     want = DeviceBatch([near]).energy_terms()
     assert torch.equal(b.energy_terms(), want)
+
+
+def test_terms_of_many_small_systems_equal_each_alone():
+    """Many small systems are summed by a CTA each, one alone by a cluster of
+    eight: the same shares in the same order, so the same bits, with atom
+    counts on both sides of a share (256) and of a round of shares (2,048)."""
+    from conftest import Golden
+    from protein_physics_b200.device import DeviceBatch
+    from protein_physics_b200.topology import flatten
+    g = Golden("insulin")
+    rng = np.random.default_rng(8)
+    sizes = [1, 255, 256, 257, 700, 2047, 2048, 2049, 2305]
+    one = (g["xyz"], g["q"], g["r"], g["eps"], flatten(g.topology()))
+    systems = [(rng.uniform(0, 10 + n ** (1 / 3) * 3, (n, 3)), rng.choice([-0.3, 0.3], n), np.full(n, 1.6),
+                np.full(n, 0.1), None) for n in sizes] + [one] * 45
+    b = DeviceBatch(systems)
+    assert b.natoms <= 16 * b.nsys ** 2
+    terms = b.energy_terms()
+    for s in range(len(sizes) + 1):
+        assert torch.equal(DeviceBatch([systems[s]]).energy_terms()[0], terms[s]), s
+    assert torch.equal(terms[-1], terms[len(sizes)])
