@@ -60,3 +60,15 @@ def test_matrices_at_tile_and_stage_edges(n_snaps, n_ca):
     f = (np.sqrt(((c[:, :, None, :] - c[:, None, :, :]) ** 2).sum(-1)) < 8.0).mean(0)
     np.fill_diagonal(f, 0.0)
     np.testing.assert_allclose(analysis.compute_contact_freq_matrix(c, 8.0), f, rtol=1e-15, atol=1e-15)
+
+
+@pytest.mark.parametrize("n_snaps,n_ca", [(1, 447), (3, 448), (4, 449), (5, 463), (9, 513)])
+def test_contacts_at_the_wide_tile_edges(n_snaps, n_ca):
+    """Contact frequencies on both sides of the residue count from which a
+    thread takes four cells, and around its 64 rows and four staged snapshots."""
+    from protein_physics_b200 import analysis
+    c = np.random.default_rng(n_ca).normal(size=(n_snaps, n_ca, 3)) * 12.0
+    f = (np.sqrt(((c[:, :, None, :] - c[:, None, :, :]) ** 2).sum(-1)) < 8.0).mean(0)
+    np.fill_diagonal(f, 0.0)
+    np.testing.assert_allclose(analysis.compute_contact_freq_matrix(c, 8.0), f, rtol=1e-15, atol=1e-15)
+    np.testing.assert_allclose(analysis.compute_mean_dist_matrix(c), _numpy_mean(c), rtol=1e-12, atol=1e-12)
