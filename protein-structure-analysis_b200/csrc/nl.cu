@@ -258,12 +258,15 @@ nl_order_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, cons
 //          tests bit for bit
 //   write  space from the system's counters (one atomic per row kind, which
 //          are also the entry counts), then the four rows, ballot-compacted
-// Issue bounds it (69 % active with 28 warps per SM, 36 fit).  The scan before this one compacted every chunk of 27 separate
-// cells as it went, about 12,000 issue slots per atom at 600 neighbours.  65k
-// atoms: 1,010 -> 431 us; 48 x 4.8k atoms: 1,892 -> 926 us.  Rows sit in their system's region in any order; a row that
+// Issue bounds it (69 % active with 28 warps per SM).  Shared memory lets eight
+// blocks, 32 warps, on an SM; the launch bound of nine caps the registers at 56,
+// 0.5 % faster than the 64 that eight would allow.  The scan before this one
+// compacted every chunk of 27 separate cells as it went, about 12,000 issue
+// slots per atom at 600 neighbours.  65k atoms: 1,010 -> 438 us; 48 x 4.8k atoms:
+// 1,892 -> 952 us.  Rows sit in their system's region in any order; a row that
 // would overflow it is not written and raises the flag.
-constexpr int NL_STAGE = 1280;  // staged entries of a row; a longer one is scanned in FP64
-constexpr int NL_CHUNKS = 160;  // chunks of 32 candidates that hold one within reach; likewise
+constexpr int NL_STAGE = 1280;  // staged entries of a row; a longer one is staged in parts
+constexpr int NL_CHUNKS = 160;  // chunks of 32 candidates that hold one within reach; a row with more is scanned in FP64
 constexpr int NL_WARPS = 4;
 constexpr uint32_t NL_SHORT_BIT = 0x40000000u;  // staging only: the pair is within SASA reach
 constexpr uint32_t NL_DROPPED = 0xffffffffu;    // staging only: not an entry (2^30 - 2 is the largest index)
@@ -301,7 +304,7 @@ __device__ __forceinline__ void set_rows(const AlmaNL &nl, int i, int n, int lan
     }
 }
 
-template <int G>
+template <int G>  // 1 or 2 atoms per warp
 __global__ void __launch_bounds__(NL_WARPS * 32, 9)
 nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const uint8_t *__restrict__ mask,
                const double *__restrict__ xyz, double rcut2, const SysGrid *__restrict__ grid,
@@ -374,7 +377,9 @@ nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const
         }
         const int total = __shfl_sync(0xffffffffu, upto, 8);
         const unsigned lt = (1u << lane) - 1u;
-        int nch = 0;
+        int nch = 0, ncand[G];  // chunks kept; this lane's candidates of each atom
+#pragma unroll
+        for (int a = 0; a < G; ++a) ncand[a] = 0;
         for (int c0 = 0; c0 < total; c0 += 32) {
             // this lane's chunk: where it starts and which of its lanes exist
             int from = 0, left = 0;
@@ -409,7 +414,10 @@ nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const
             const uint32_t exist = left >= 32 ? 0xffffffffu : left > 0 ? (1u << left) - 1u : 0u;
             uint32_t any = 0u;
 #pragma unroll
-            for (int a = 0; a < G; ++a) any |= keep[a] &= exist;
+            for (int a = 0; a < G; ++a) {
+                any |= keep[a] &= exist;
+                ncand[a] += __popc(keep[a]);
+            }
             const unsigned some = __ballot_sync(0xffffffffu, any != 0u);
             const int at = nch + __popc(some & lt);
             if (any != 0u && at < NL_CHUNKS) {
@@ -426,27 +434,8 @@ nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const
             const int i = __shfl_sync(0xffffffffu, my_i, a);
             const double4 pi = ld_xyz(xyz, i);
             const double ri_pad = shorts ? prm64[4 * (size_t)i + 1] + reach_pad : 0.0;
-            int n = nch <= NL_CHUNKS ? 0 : NL_STAGE + 1;
-            for (int b = 0; b < nch && n <= NL_STAGE; b += 32) {
-                uint32_t m = b + lane < nch ? W.bits[a][b + lane] : 0u;
-                const int32_t from = b + lane < nch ? W.base[b + lane] : 0;
-                const int cnt = __popc(m);
-                int inc = cnt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int u = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += u;
-                }
-                int at = n + inc - cnt;
-                n += __shfl_sync(0xffffffffu, inc, 31);
-                if (n <= NL_STAGE)
-                    while (m) {
-                        W.stage[at++] = (uint32_t)(from + __ffs(m) - 1);
-                        m &= m - 1u;
-                    }
-            }
-            int64_t off = 0;
-            if (n > NL_STAGE) {  // too long to stage: counted, then written, by FP64 scans
+            if (nch > NL_CHUNKS) {  // too many chunks to list: counted, then written, by FP64 scans
+                int64_t off = 0;
                 int c[4];
                 nl_row_atom<0>(i, lane, g, xyz, rcut2, cell_of, cells, cell_atoms, prm64, reach_pad, excl_ptr,
                                excl_cols, excl_win, nl, c[0], c[1], c[2], c[3]);
@@ -459,57 +448,88 @@ nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const
                 }
                 continue;
             }
-            __syncwarp();
             const float4 pf = cell_atom[p0 + a];
             const float rpad_f = (float)ri_pad;
             const uint4 ew = excl_window_of(excl_win, i);
             int cf = 0, cs = 0;  // this lane's entries: full | half << 16, short full | short half << 16
             int jmin = 0x7fffffff, jmax = -1;
-#pragma unroll 2
-            for (int t = lane; t < n; t += 32) {
-                const int k = (int)W.stage[t];
-                const int j = cell_atoms[k];
-                const float4 q = cell_atom[k];
-                const float dx = q.x - pf.x, dy = q.y - pf.y, dz = q.z - pf.z;
-                const float r2f = dx * dx + dy * dy + dz * dz;
-                uint32_t e = NL_DROPPED;
-                if (r2f < cut_hi && j != i) {
-                    double r2 = -1.0;  // FP64 r², computed only when a test needs it
-                    bool in = true, sh = false;
-                    if (r2f > cut_lo) {
-                        r2 = d2_of(pi, ld_xyz(xyz, j));
-                        in = r2 < rcut2;
+            // chunks [b0, b1): candidates listed, then decided in place
+            auto stage = [&](int b0, int b1) {
+                int n = 0;
+                __syncwarp();  // the entries staged before have been read
+                for (int b = b0; b < b1; b += 32) {
+                    uint32_t m = b + lane < b1 ? W.bits[a][b + lane] : 0u;
+                    const int32_t from = b + lane < b1 ? W.base[b + lane] : 0;
+                    const int cnt = __popc(m);
+                    int inc = cnt;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int u = __shfl_up_sync(0xffffffffu, inc, o);
+                        if (lane >= o) inc += u;
                     }
-                    if (in && shorts) {
-                        const float rf = rpad_f + q.w, rf2 = rf * rf;
-                        if (r2f < rf2 - m2) {
-                            sh = true;
-                        } else if (r2f <= rf2 + m2) {
-                            if (r2 < 0.0) r2 = d2_of(pi, ld_xyz(xyz, j));
-                            const double reach = ri_pad + prm64[4 * (size_t)j + 1];
-                            sh = r2 < reach * reach;
-                        }
-                    }
-                    if (in) {
-                        e = (uint32_t)j |
-                            (excluded_w(excl_win, ew, excl_ptr, excl_cols, i, j) ? ALMA_EXCL_BIT : 0u) |
-                            (sh ? NL_SHORT_BIT : 0u);
-                        const int up = j > i ? 0x10001 : 1;
-                        cf += up;
-                        cs += sh ? up : 0;
-                        jmin = min(jmin, j);
-                        jmax = max(jmax, j);
+                    int at = n + inc - cnt;
+                    n += __shfl_sync(0xffffffffu, inc, 31);
+                    while (m) {
+                        W.stage[at++] = (uint32_t)(from + __ffs(m) - 1);
+                        m &= m - 1u;
                     }
                 }
-                W.stage[t] = e;
-            }
+                __syncwarp();
+#pragma unroll 2
+                for (int t = lane; t < n; t += 32) {
+                    const int k = (int)W.stage[t];
+                    const int j = cell_atoms[k];
+                    const float4 q = cell_atom[k];
+                    const float dx = q.x - pf.x, dy = q.y - pf.y, dz = q.z - pf.z;
+                    const float r2f = dx * dx + dy * dy + dz * dz;
+                    uint32_t e = NL_DROPPED;
+                    if (r2f < cut_hi && j != i) {
+                        double r2 = -1.0;  // FP64 r², computed only when a test needs it
+                        bool in = true, sh = false;
+                        if (r2f > cut_lo) {
+                            r2 = d2_of(pi, ld_xyz(xyz, j));
+                            in = r2 < rcut2;
+                        }
+                        if (in && shorts) {
+                            const float rf = rpad_f + q.w, rf2 = rf * rf;
+                            if (r2f < rf2 - m2) {
+                                sh = true;
+                            } else if (r2f <= rf2 + m2) {
+                                if (r2 < 0.0) r2 = d2_of(pi, ld_xyz(xyz, j));
+                                const double reach = ri_pad + prm64[4 * (size_t)j + 1];
+                                sh = r2 < reach * reach;
+                            }
+                        }
+                        if (in) {
+                            e = (uint32_t)j |
+                                (excluded_w(excl_win, ew, excl_ptr, excl_cols, i, j) ? ALMA_EXCL_BIT : 0u) |
+                                (sh ? NL_SHORT_BIT : 0u);
+                            const int up = j > i ? 0x10001 : 1;
+                            cf += up;
+                            cs += sh ? up : 0;
+                            jmin = min(jmin, j);
+                            jmax = max(jmax, j);
+                        }
+                    }
+                    W.stage[t] = e;
+                }
+                return n;
+            };
+            // A row that fits the stage goes through it whole; a longer one 32
+            // chunks at a time, once to be counted and again to be written.  48
+            // chains of 4,962 atoms scaled to 0.9, where one row in six is longer:
+            // 2,441 us, 3,953 with FP64 scans of the 27 cells for those.
+            int64_t off = 0;
+            uint32_t *wf = nullptr, *wh = nullptr, *wsf = nullptr, *wsh = nullptr;
+            const int listed = __reduce_add_sync(0xffffffffu, G > 1 && a > 0 ? ncand[G - 1] : ncand[0]);
+            const int step = listed <= NL_STAGE ? NL_CHUNKS : 32;
+            int n = 0;
+#pragma unroll 1
+            for (int b = 0; b < nch; b += step) n = stage(b, min(nch, b + step));
             cf = __reduce_add_sync(0xffffffffu, cf);
             cs = __reduce_add_sync(0xffffffffu, cs);
             const int cnt = lane == 0 ? cf & 0xffff : lane == 1 ? cf >> 16 : lane == 2 ? cs & 0xffff : cs >> 16;
-            if (!take_rows(nl, s, cnt, lane, nkind, off, status)) {
-                __syncwarp();
-                continue;
-            }
+            if (!take_rows(nl, s, cnt, lane, nkind, off, status)) continue;
             set_rows(nl, i, cnt, lane, nkind, off);
             if (lane == 0) *reinterpret_cast<double4 *>(nl.ref_xyz + 4 * (size_t)i) = pi;
             if (nl.full_span != nullptr) {
@@ -520,33 +540,39 @@ nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const
                     nl.full_span[2 * (size_t)i + 1] = jmax;
                 }
             }
-            uint32_t *wf = nl.full_cols + __shfl_sync(0xffffffffu, off, 0);
-            uint32_t *wh = nl.half_cols + __shfl_sync(0xffffffffu, off, 1);
-            uint32_t *wsf = shorts ? nl.sfull_cols + __shfl_sync(0xffffffffu, off, 2) : nullptr;
-            uint32_t *wsh = shorts ? nl.shalf_cols + __shfl_sync(0xffffffffu, off, 3) : nullptr;
-            for (int t0 = 0; t0 < n; t0 += 32) {
-                const uint32_t st = t0 + lane < n ? W.stage[t0 + lane] : NL_DROPPED;
-                const bool v = st != NL_DROPPED;
-                const bool hf = v && (int)(st & (ALMA_IDX_MASK & ~NL_SHORT_BIT)) > i;
-                const unsigned mf = __ballot_sync(0xffffffffu, v), mh = __ballot_sync(0xffffffffu, hf);
-                const uint32_t e = st & ~NL_SHORT_BIT;
-                if (v) wf[__popc(mf & lt)] = e;
-                if (hf) wh[__popc(mh & lt)] = e;
-                wf += __popc(mf);
-                wh += __popc(mh);
-                if (shorts) {
-                    const bool sh = v && (st & NL_SHORT_BIT);
-                    const unsigned ms = __ballot_sync(0xffffffffu, sh), msh = ms & mh;
-                    if (sh) {
-                        wsf[__popc(ms & lt)] = e;
-                        if (hf) wsh[__popc(msh & lt)] = e;
+            wf = nl.full_cols + __shfl_sync(0xffffffffu, off, 0);
+            wh = nl.half_cols + __shfl_sync(0xffffffffu, off, 1);
+            if (shorts) {
+                wsf = nl.sfull_cols + __shfl_sync(0xffffffffu, off, 2);
+                wsh = nl.shalf_cols + __shfl_sync(0xffffffffu, off, 3);
+            }
+#pragma unroll 1
+            for (int b = 0; b < nch; b += step) {
+                if (step < NL_CHUNKS) n = stage(b, min(nch, b + step));
+                for (int t0 = 0; t0 < n; t0 += 32) {
+                    const uint32_t st = t0 + lane < n ? W.stage[t0 + lane] : NL_DROPPED;
+                    const bool v = st != NL_DROPPED;
+                    const bool hf = v && (int)(st & (ALMA_IDX_MASK & ~NL_SHORT_BIT)) > i;
+                    const unsigned mf = __ballot_sync(0xffffffffu, v), mh = __ballot_sync(0xffffffffu, hf);
+                    const uint32_t e = st & ~NL_SHORT_BIT;
+                    if (v) wf[__popc(mf & lt)] = e;
+                    if (hf) wh[__popc(mh & lt)] = e;
+                    wf += __popc(mf);
+                    wh += __popc(mh);
+                    if (shorts) {
+                        const bool sh = v && (st & NL_SHORT_BIT);
+                        const unsigned ms = __ballot_sync(0xffffffffu, sh), msh = ms & mh;
+                        if (sh) {
+                            wsf[__popc(ms & lt)] = e;
+                            if (hf) wsh[__popc(msh & lt)] = e;
+                        }
+                        wsf += __popc(ms);
+                        wsh += __popc(msh);
                     }
-                    wsf += __popc(ms);
-                    wsh += __popc(msh);
                 }
             }
-            __syncwarp();  // the stage is the next atom's
         }
+        __syncwarp();  // the masks and the stage are the next atoms'
     }
 }
 
@@ -638,8 +664,8 @@ extern "C" int alma_nl_build(const AlmaBatch *b, const AlmaTopo *t, AlmaNL *nl, 
     const uint32_t *ew = t && t->excl_ptr ? t->excl_win : nullptr;
     // Two atoms per warp read each candidate once for both; below about two
     // waves of one-atom warps the chip has room for the shorter chains (16k
-    // atoms: 95 us with one, 98 with two; 32k: 203 and 194; 65k: 481 and 445;
-    // four per warp: 125, 222 and 474).
+    // atoms: 96 us with one, 97 with two; 24k: 160 and 152; 32k: 178 and 170; 65k:
+    // 492 and 438).
     auto rows = [&](auto kfn, int per_warp) {
         const int per_block = per_warp * NL_WARPS;
         kfn<<<(natoms + per_block - 1) / per_block, NL_WARPS * 32, 0, st>>>(

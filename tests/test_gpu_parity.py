@@ -522,3 +522,27 @@ def test_terms_of_many_small_systems_equal_each_alone():
     for s in range(len(sizes) + 1):
         assert torch.equal(DeviceBatch([systems[s]]).energy_terms()[0], terms[s]), s
     assert torch.equal(terms[-1], terms[len(sizes)])
+
+
+@pytest.mark.parametrize("copies", [1, 10])
+def test_nl_rows_past_the_stage(oracle, copies):
+    """Rows of more candidates than the stage holds, listed in 2 to 5 groups of 32
+    chunks, with one atom per warp and with two (24,000 atoms and more): half
+    rows equal to the oracle's, order included, full rows in their order."""
+    from protein_physics_b200.device import DeviceBatch
+    x = np.random.default_rng(21).uniform(0, 17, (2600, 3))
+    b = DeviceBatch([(x, np.zeros(len(x)), np.full(len(x), 1.9), np.full(len(x), 0.1), None)] * copies)
+    assert (b.natoms >= 24000) == (copies == 10)
+    b.build_nl()
+    ptr, ocols = oracle.nl_build(x)
+    for s in {0, copies - 1}:
+        rp, cols, _ = b.nl_host(s, half=True)
+        assert np.array_equal(rp, ptr) and np.array_equal(cols, ocols), s
+        frp, fcols, _ = b.nl_host(s, half=False)
+        J = np.repeat(np.arange(len(x)), np.diff(frp))
+        assert np.diff(frp).max() > 1536 and len(fcols) == 2 * len(ocols)
+        assert np.array_equal(fcols[fcols > J], ocols), s
+        srp, scols, _ = b.nl_host(s, half=False, short=True)
+        r2 = ((x[J] - x[fcols]) ** 2).sum(1)
+        reach = 2 * 1.9 + 2 * b.params.probe_r + 2 * np.sqrt(b.params.half_skin2) + 1e-6
+        assert np.array_equal(scols, fcols[r2 < reach * reach]), s
