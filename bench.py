@@ -265,8 +265,7 @@ def _kernel_roofline(runner, batch, tuned, proposals_per_launch, workload=None):
     d = c1 - c0
     ops = d[0] * OPS_PAIR + d[1] * OPS_HCT + d[2] * OPS_SASA
     achieved = ops / (k_ms * 1e-3)
-    # CTA size 0: chosen by the library from the atoms per CTA
-    threads = tuned[1] or (1024 if batch.natoms >= 256 * tuned[0] * batch.nsys else 512)
+    threads = tuned[1] or batch.L.alma_mc_cta_threads(batch.natoms, batch.nsys, tuned[0], batch.prec)
     name = ("mc_spec_kernel<float,%d,%d> x %d teams" % (threads, tuned[0], tuned[2]) if tuned[2] > 1 else
             "mc_kernel<float,%d,%d>" % (threads, tuned[0]))
     nprop = float(np.sum(st1["step"] - st0["step"]))

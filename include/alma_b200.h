@@ -454,6 +454,9 @@ size_t alma_mc_rebuild_bytes(int32_t natoms, int32_t nsys);
 /* Scratch bytes of alma_mc_run for spec_teams = teams (zeroed once before
  * first use; teams <= 1: alma_move_scratch_bytes(natoms)). */
 size_t alma_mc_scratch_bytes(int32_t natoms, int32_t nsys, int32_t teams);
+/* CTA size alma_mc_run takes for threads_per_system = 0 on a batch of nsys
+ * systems of natoms atoms together: 512 or 1024. */
+int alma_mc_cta_threads(int32_t natoms, int32_t nsys, int32_t cluster_size, int prec);
 /* Runs proposals on every system until its state.step reaches step_limit
  * or it needs a neighbor-list rebuild (one CTA per system, no host sync).
  * The caller then rebuilds flagged systems (alma_nl_build + alma_born_radii

@@ -804,6 +804,21 @@ int alma_check_move_args(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *nl
 MoveCtx alma_make_move_ctx(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *nl, const AlmaParams *p,
                            void *scratch);
 
+// 1,024 threads at 64 registers hide the latency of the row scans better than 512
+// at 128, in spite of some spilled registers, where an average system has an
+// atom for every four threads or more; with less the barriers of twice the
+// warps cost more than that.  One team, 512 / 1,024 threads, us a proposal, 4
+// chains: 64 residues on 1, 4, 8, 16 CTAs (1,089 to 68 atoms each) 352 / 281,
+// 147 / 137, 112 / 115, 100 / 115; 300 residues on 4, 16 CTAs 380 / 304, 161 /
+// 156.  256 chains of 50-600 residues on 4-CTA clusters, 50 proposals: 169 / 132
+// ms.  256 threads are slower everywhere (600 chains of 30 residues: 1,096 / 746 /
+// 638 us).  Four teams of 16 CTAs: 63 / 60 us for 4.9k atoms, 26 / 28 for 1.1k.
+// FP64 pair terms need the registers.
+extern "C" int alma_mc_cta_threads(int32_t natoms, int32_t nsys, int32_t cluster_size, int prec) {
+    const int64_t cl = cluster_size <= 0 ? 1 : cluster_size;
+    return prec != ALMA_PREC_FP64 && (int64_t)natoms >= 256 * cl * nsys ? 1024 : 512;
+}
+
 extern "C" int alma_mc_run(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *nl, const AlmaParams *p, int prec,
                            void *scratch, const AlmaMCConfig *cfg, AlmaChainState *states, int64_t step_limit,
                            void *stream) {
@@ -838,21 +853,11 @@ extern "C" int alma_mc_run(const AlmaBatch *b, const AlmaTopo *t, const AlmaNL *
     cudaStream_t st = (cudaStream_t)stream;
     const int cl = cfg->cluster_size <= 0 ? 1 : cfg->cluster_size;
     // cluster_size CTAs cooperate on each system (1, 2, 4, 8 or 16), one CTA
-    // per SM.  Threads per CTA: the caller's choice, or by size.  1,024 at 64
-    // registers hide the latency of the row scans better than 512 at 128, in
-    // spite of some spilled registers, where an average system has an atom for
-    // every four threads or more; with less the barriers of twice the warps cost
-    // more than that.  One team, 512 / 1,024 threads, us a proposal, 4 chains:
-    // 64 residues on 1, 4, 8, 16 CTAs (1,089 to 68 atoms each) 352 / 281,
-    // 147 / 137, 112 / 115, 100 / 115; 300 residues on 4, 16 CTAs 380 / 304,
-    // 161 / 156.  256 chains of 50-600 residues on 4-CTA clusters, 50
-    // proposals: 169 / 132 ms.  256 threads are slower everywhere (600 chains of
-    // 30 residues: 1,096 / 746 / 638 us).  Four teams of 16 CTAs: 63 / 60 us
-    // for 4.9k atoms, 26 / 28 for 1.1k.  FP64 pair terms need the registers.
+    // per SM.  Threads per CTA: the caller's choice, or by size.
     int nt = cfg->threads_per_system;
     if (nt != 0 && nt != 256 && nt != 512)
         return alma_set_error(ALMA_EINVAL, "alma_mc_run: threads_per_system must be 0, 256 or 512");
-    if (nt == 0) nt = prec != ALMA_PREC_FP64 && (int64_t)b->natoms >= (int64_t)256 * cl * b->nsys ? 1024 : 512;
+    if (nt == 0) nt = alma_mc_cta_threads(b->natoms, b->nsys, cl, prec);
     if (cl != 1 && cl != 2 && cl != 4 && cl != 8 && cl != 16)
         return alma_set_error(ALMA_EINVAL, "alma_mc_run: cluster_size must be 1, 2, 4, 8 or 16");
     const int teams = cfg->spec_teams <= 1 ? 1 : cfg->spec_teams;

@@ -135,6 +135,8 @@ def lib():
     L.alma_move_scratch_bytes.argtypes = [_i32]
     L.alma_mc_scratch_bytes.restype = C.c_size_t
     L.alma_mc_scratch_bytes.argtypes = [_i32, _i32, _i32]
+    L.alma_mc_cta_threads.restype = C.c_int
+    L.alma_mc_cta_threads.argtypes = [_i32, _i32, _i32, C.c_int]
     L.alma_mc_rebuild_bytes.restype = C.c_size_t
     L.alma_mc_rebuild_bytes.argtypes = [_i32, _i32]
     L.alma_spec_round_bytes.restype = C.c_size_t

@@ -251,22 +251,41 @@ class MCRunner:
 _TUNED = {}
 
 
+def _tune_key(batch, policy, moveset):
+    """What a tuned shape is kept under: the number of systems, their mean
+    atoms and how far the largest is from the mean (powers of two), the
+    precision (the CTA size rule follows it) and the proposals."""
+    sizes = np.maximum(np.diff(batch.atom_off_h), 1)
+    mean = max(1, batch.natoms // max(1, batch.nsys))
+    return (batch.nsys, int(np.log2(mean)), int(np.log2(max(1.0, sizes.max() / mean))), batch.prec, policy,
+            moveset is not None)
+
+
+def _tune_candidates(batch, sms):
+    """(cluster size, threads, teams) to try: the library's CTA size (0) and,
+    where that is 1,024, 512 threads (256 are slower on every shape)."""
+    nsys = batch.nsys
+    wide = max(2 * sms, 8 * nsys if 2 * nsys > sms else 0)  # queued systems: up to 8-CTA clusters
+    shapes = [(cl, 1) for cl in (1, 2, 4, 8, 16) if nsys * cl <= wide]
+    shapes += [(cl, k) for cl in (8, 16) for k in (2, 4, 8) if nsys * cl * k <= sms]
+    rule = _lib.lib().alma_mc_cta_threads
+    return [(cl, nt, k) for cl, k in shapes
+            for nt in ((0, 512) if rule(batch.natoms, nsys, cl, batch.prec) > 512 else (0,))]
+
+
 def autotune(batch, temperatures, seed, policy=0, moveset=None, proposals=200, candidates=None):
     """Picks (cluster_size, threads_per_system, spec_teams) for this batch shape by
     timing `proposals` proposals per candidate, after as many untimed ones
     (the step scale and the acceptance rate, on which the speculative teams'
     gain depends, settle first), on a scratch copy of the batch state;
-    cached per (systems, atom-count bucket, policy)."""
+    cached per kind of batch (_tune_key)."""
     import time
     sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
-    key = (batch.nsys, int(np.log2(max(1, batch.natoms // max(1, batch.nsys)))), policy, moveset is not None)
+    key = _tune_key(batch, policy, moveset)
     if key in _TUNED:
         return _TUNED[key]
     if candidates is None:
-        wide = max(2 * sms, 8 * batch.nsys if 2 * batch.nsys > sms else 0)  # queued systems: up to 8-CTA clusters
-        candidates = [(cl, nt, 1) for cl in (1, 2, 4, 8, 16) for nt in (0, 512) if batch.nsys * cl <= wide]
-        candidates += [(cl, nt, k) for cl in (8, 16) for nt in (0, 512) for k in (2, 4, 8)
-                       if batch.nsys * cl * k <= sms]
+        candidates = _tune_candidates(batch, sms)
     xyz0, born0 = batch.xyz.clone(), batch.born.clone()
     best, best_rate = None, -1.0
     for cand in candidates:

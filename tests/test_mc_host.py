@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from protein_physics_b200 import _lib
-from protein_physics_b200.mc import TAIL_MAX_TEAMS, MCRunner, auto_shape
+from protein_physics_b200.mc import TAIL_MAX_TEAMS, MCRunner, _tune_candidates, _tune_key, auto_shape
 
 
 @pytest.mark.parametrize("sms", [148, 132])
@@ -83,3 +83,41 @@ def test_auto_shape_of_queued_systems_balances_the_longest_chain():
             assert cl == 1 or sizes.max() / (cl // 2) > 0.4 * share
     assert auto_shape(74, 148, np.full(74, 5000)) == (2, 1)
     assert auto_shape(256, 148, np.linspace(800, 9800, 256)) == (4, 1)
+
+
+@pytest.mark.parametrize("cluster", [1, 2, 4, 8, 16])
+def test_cta_size_rule(cluster):
+    """1,024 threads from 256 atoms per CTA of the mean system on, in mixed
+    precision; FP64 always takes 512."""
+    rule = _lib.lib().alma_mc_cta_threads
+    for nsys in (1, 3, 400):
+        line = 256 * cluster * nsys
+        assert rule(line, nsys, cluster, _lib.PREC_MIXED) == 1024
+        assert rule(line - 1, nsys, cluster, _lib.PREC_MIXED) == 512
+        assert rule(line, nsys, cluster, _lib.PREC_FP64) == 512
+
+
+def _batch(sizes, prec=_lib.PREC_MIXED):
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    return types.SimpleNamespace(atom_off_h=off, nsys=len(sizes), natoms=int(off[-1]), prec=prec)
+
+
+def test_tuned_shapes_are_kept_per_precision_and_spread():
+    even, fp64 = _batch([1000] * 32), _batch([1000] * 32, _lib.PREC_FP64)
+    uneven = _batch([516] * 31 + [16004])
+    keys = [_tune_key(b, 0, None) for b in (even, fp64, uneven)]
+    assert len(set(keys)) == 3
+    assert _tune_key(_batch([1010] * 32), 0, None) == keys[0]
+    assert _tune_key(even, 0, [[0]] * 32) != keys[0] != _tune_key(even, 1, None)
+
+
+@pytest.mark.parametrize("sizes", [[1000], [300] * 40, [5000] * 200])
+def test_tune_candidates_name_each_kernel_once(sizes):
+    rule = _lib.lib().alma_mc_cta_threads
+    for prec in (_lib.PREC_MIXED, _lib.PREC_FP64):
+        b = _batch(sizes, prec)
+        found = _tune_candidates(b, 148)
+        real = [(cl, nt or rule(b.natoms, b.nsys, cl, prec), k) for cl, nt, k in found]
+        assert len(set(real)) == len(real)
+        assert prec != _lib.PREC_FP64 or all(nt == 512 for _, nt, _ in real)
+        assert {(cl, k) for cl, _, k in found} >= {(1, 1), (2, 1)}
