@@ -350,13 +350,13 @@ __device__ bool team_rebuild(const MoveCtx &C, const MCConfigDev &cfg, int s, co
 // and decisions (the ΔE totals are bit-identical in every CTA); rank 0
 // writes the state back.
 //
-// One CTA per SM is all the launches ask for, and said so in the bounds: 512
-// threads then get up to 128 registers, where the compiler by itself stops at
-// 64 and spills 0.6-1.1 KB (40 FP64 chains of 300 residues on 2-CTA clusters:
-// 2,340 us a proposal at 64 registers, 1,942 here).
-template <typename R, int NT, int CL>
-__global__ void __launch_bounds__(NT, 1) mc_kernel(MoveCtx C, MCConfigDev cfg,
-                                                   AlmaChainState *__restrict__ states, int64_t step_limit) {
+// SHARE CTAs per SM.  One is what nearly every launch asks for, and 512 threads
+// then get up to 128 registers, where the compiler by itself stops at 64 and
+// spills 0.6-1.1 KB (40 FP64 chains of 300 residues on 2-CTA clusters: 2,340 us
+// a proposal at 64 registers, 1,942 at 128).  Two, at 64: see launch_mc.
+template <typename R, int NT, int CL, int SHARE>
+__global__ void __launch_bounds__(NT, SHARE) mc_kernel(MoveCtx C, MCConfigDev cfg,
+                                                       AlmaChainState *__restrict__ states, int64_t step_limit) {
     __shared__ MoveDesc M;
     __shared__ double sm[128];
     __shared__ double part[8];
@@ -450,7 +450,7 @@ static size_t warp_smem_bytes(int nt) {
 template <typename R, int NT, int CL>
 static cudaError_t launch_mc(const MoveCtx &C, const MCConfigDev &d, AlmaChainState *states, int64_t step_limit,
                              int nsys, int nt, cudaStream_t st) {
-    auto kfn = mc_kernel<R, NT, CL>;
+    auto kfn = mc_kernel<R, NT, CL, 1>;
     const size_t smem = warp_smem_bytes(nt);
     if (NT > 512) {  // past the 48 KB that need no opt-in
         cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -460,10 +460,6 @@ static cudaError_t launch_mc(const MoveCtx &C, const MCConfigDev &d, AlmaChainSt
         kfn<<<nsys, nt, smem, st>>>(C, d, states, step_limit);
         return cudaGetLastError();
     } else {
-        if (CL > 8) {
-            cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            if (e != cudaSuccess) return e;
-        }
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(nsys * CL), 1, 1);
         cfg.blockDim = dim3((unsigned)nt, 1, 1);
@@ -476,10 +472,32 @@ static cudaError_t launch_mc(const MoveCtx &C, const MCConfigDev &d, AlmaChainSt
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
+        auto resident = [&](auto k, int &clusters) {
+            if (CL > 8) {
+                const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+                if (e != cudaSuccess) return e;
+            }
+            return cudaOccupancyMaxActiveClusters(&clusters, k, &cfg);
+        };
         int max_clusters = 0;
-        cudaError_t e = cudaOccupancyMaxActiveClusters(&max_clusters, kfn, &cfg);
+        cudaError_t e = resident(kfn, max_clusters);
         if (e != cudaSuccess) return e;
         if (max_clusters < 1) return cudaErrorInvalidConfiguration;  // cluster does not fit a GPC
+        // A chain that rebuilds its own list holds its SMs for the whole run, so a
+        // cluster that finds no room waits for a whole chain: two CTAs then share
+        // an SM.  One per SM, 33 clusters of 4 CTAs, 15 of 8 and 7 of 16 fit.  64
+        // residues, 200 proposals, one per SM / two: 16 chains on 8 CTAs 24.7 / 20.6
+        // ms, 8 chains on 16 CTAs 20.8 / 15.9; with room for all one is faster (12
+        // chains on 8 CTAs 15.9 / 17.6).
+        if constexpr (NT == 512) {
+            if (d.rw.ccount && max_clusters < nsys) {
+                auto shared = mc_kernel<R, NT, CL, 2>;
+                int both = 0;
+                e = resident(shared, both);
+                if (e != cudaSuccess) return e;
+                if (both >= nsys) return cudaLaunchKernelEx(&cfg, shared, C, d, states, step_limit);
+            }
+        }
         return cudaLaunchKernelEx(&cfg, kfn, C, d, states, step_limit);
     }
 }

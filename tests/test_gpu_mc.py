@@ -332,3 +332,21 @@ def test_threads_by_size_make_the_same_chain(cluster, teams, precision):
         assert (acc, reb) == out[0][1:3]
         np.testing.assert_array_equal(x, out[0][0])
         assert e == pytest.approx(out[0][3], rel=1e-10, abs=1e-8)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("nsys,cluster", [(16, 8), (8, 16)])
+def test_clusters_that_share_sms_make_the_same_chains(nsys, cluster, precision):
+    """More clusters than fit at one CTA per SM, each rebuilding its own lists:
+    two CTAs share an SM then, on a kernel with half the registers.  The chains
+    are those of the kernel that has the SM to itself (host rebuilds): decisions,
+    and coordinates to the bit; the energies differ by the order of FP64 sums."""
+    g, F = _setup("insulin")
+    kw = dict(precision=precision, cluster_size=cluster, spec_teams=1, tail_shape=False, fixed_delta=0.3, T=10.0)
+    b1, st1 = _gpu_run(g, F, nsys, 13, 60, device_rebuild=True, **kw)
+    b2, st2 = _gpu_run(g, F, nsys, 13, 60, device_rebuild=False, **kw)
+    assert st1["n_rebuild"].sum() > 0
+    for s in range(nsys):
+        assert st1["n_accepted"][s] == st2["n_accepted"][s]
+        assert np.array_equal(b1.coords(s), b2.coords(s)), s
+        assert st1["energy"][s] == pytest.approx(st2["energy"][s], rel=1e-9)
