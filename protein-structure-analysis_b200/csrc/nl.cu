@@ -258,15 +258,13 @@ nl_order_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, cons
 //          tests bit for bit
 //   write  space from the system's counters (one atomic per row kind, which
 //          are also the entry counts), then the four rows, ballot-compacted
-// Issue bounds it (69 % active with 28 warps per SM).  Shared memory lets eight
-// blocks, 32 warps, on an SM; the launch bound of nine caps the registers at 56,
-// 0.5 % faster than the 64 that eight would allow.  The scan before this one
-// compacted every chunk of 27 separate cells as it went, about 12,000 issue
-// slots per atom at 600 neighbours.  65k atoms: 1,010 -> 438 us; 48 x 4.8k atoms:
-// 1,892 -> 952 us.  Rows sit in their system's region in any order; a row that
-// would overflow it is not written and raises the flag.
+// Issue bounds it; shared memory lets eight blocks, 32 warps, on an SM.  The scan
+// before this one compacted every chunk of 27 separate cells as it went, about
+// 12,000 issue slots per atom at 600 neighbours.  65k atoms: 1,010 -> 431 us; 48 x
+// 4.8k atoms: 1,892 -> 934 us.  Rows sit in their system's region in any order; a
+// row that would overflow it is not written and raises the flag.
 constexpr int NL_STAGE = 1280;  // staged entries of a row; a longer one is staged in parts
-constexpr int NL_CHUNKS = 160;  // chunks of 32 candidates that hold one within reach; a row with more is scanned in FP64
+constexpr int NL_CHUNKS = 160;  // chunks of 32 candidates that hold one within reach; more are scanned in FP64
 constexpr int NL_WARPS = 4;
 constexpr uint32_t NL_SHORT_BIT = 0x40000000u;  // staging only: the pair is within SASA reach
 constexpr uint32_t NL_DROPPED = 0xffffffffu;    // staging only: not an entry (2^30 - 2 is the largest index)
@@ -304,8 +302,8 @@ __device__ __forceinline__ void set_rows(const AlmaNL &nl, int i, int n, int lan
     }
 }
 
-template <int G>  // 1 or 2 atoms per warp
-__global__ void __launch_bounds__(NL_WARPS * 32, 9)
+template <int G>
+__global__ void __launch_bounds__(NL_WARPS * 32, 8)
 nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const uint8_t *__restrict__ mask,
                const double *__restrict__ xyz, double rcut2, const SysGrid *__restrict__ grid,
                const int32_t *__restrict__ cell_of, const int32_t *__restrict__ cell_end,
@@ -377,9 +375,7 @@ nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const
         }
         const int total = __shfl_sync(0xffffffffu, upto, 8);
         const unsigned lt = (1u << lane) - 1u;
-        int nch = 0, ncand[G];  // chunks kept; this lane's candidates of each atom
-#pragma unroll
-        for (int a = 0; a < G; ++a) ncand[a] = 0;
+        int nch = 0;
         for (int c0 = 0; c0 < total; c0 += 32) {
             // this lane's chunk: where it starts and which of its lanes exist
             int from = 0, left = 0;
@@ -414,10 +410,7 @@ nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const
             const uint32_t exist = left >= 32 ? 0xffffffffu : left > 0 ? (1u << left) - 1u : 0u;
             uint32_t any = 0u;
 #pragma unroll
-            for (int a = 0; a < G; ++a) {
-                any |= keep[a] &= exist;
-                ncand[a] += __popc(keep[a]);
-            }
+            for (int a = 0; a < G; ++a) any |= keep[a] &= exist;
             const unsigned some = __ballot_sync(0xffffffffu, any != 0u);
             const int at = nch + __popc(some & lt);
             if (any != 0u && at < NL_CHUNKS) {
@@ -453,11 +446,12 @@ nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const
             const uint4 ew = excl_window_of(excl_win, i);
             int cf = 0, cs = 0;  // this lane's entries: full | half << 16, short full | short half << 16
             int jmin = 0x7fffffff, jmax = -1;
-            // chunks [b0, b1): candidates listed, then decided in place
-            auto stage = [&](int b0, int b1) {
+            uint32_t *wf = nullptr, *wh = nullptr, *wsf = nullptr, *wsh = nullptr;
+            // the candidates of chunks [b0, b1) into the stage: how many, or more than
+            // NL_STAGE (and a useless stage) when they do not fit
+            auto list = [&](int b0, int b1) {
                 int n = 0;
-                __syncwarp();  // the entries staged before have been read
-                for (int b = b0; b < b1; b += 32) {
+                for (int b = b0; b < b1 && n <= NL_STAGE; b += 32) {
                     uint32_t m = b + lane < b1 ? W.bits[a][b + lane] : 0u;
                     const int32_t from = b + lane < b1 ? W.base[b + lane] : 0;
                     const int cnt = __popc(m);
@@ -469,12 +463,16 @@ nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const
                     }
                     int at = n + inc - cnt;
                     n += __shfl_sync(0xffffffffu, inc, 31);
-                    while (m) {
-                        W.stage[at++] = (uint32_t)(from + __ffs(m) - 1);
-                        m &= m - 1u;
-                    }
+                    if (n <= NL_STAGE)
+                        while (m) {
+                            W.stage[at++] = (uint32_t)(from + __ffs(m) - 1);
+                            m &= m - 1u;
+                        }
                 }
                 __syncwarp();
+                return n;
+            };
+            auto decide = [&](int n) {
 #pragma unroll 2
                 for (int t = lane; t < n; t += 32) {
                     const int k = (int)W.stage[t];
@@ -513,42 +511,30 @@ nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const
                     }
                     W.stage[t] = e;
                 }
-                return n;
             };
-            // A row that fits the stage goes through it whole; a longer one 32
-            // chunks at a time, once to be counted and again to be written.  48
-            // chains of 4,962 atoms scaled to 0.9, where one row in six is longer:
-            // 2,441 us, 3,953 with FP64 scans of the 27 cells for those.
-            int64_t off = 0;
-            uint32_t *wf = nullptr, *wh = nullptr, *wsf = nullptr, *wsh = nullptr;
-            const int listed = __reduce_add_sync(0xffffffffu, G > 1 && a > 0 ? ncand[G - 1] : ncand[0]);
-            const int step = listed <= NL_STAGE ? NL_CHUNKS : 32;
-            int n = 0;
-#pragma unroll 1
-            for (int b = 0; b < nch; b += step) n = stage(b, min(nch, b + step));
-            cf = __reduce_add_sync(0xffffffffu, cf);
-            cs = __reduce_add_sync(0xffffffffu, cs);
-            const int cnt = lane == 0 ? cf & 0xffff : lane == 1 ? cf >> 16 : lane == 2 ? cs & 0xffff : cs >> 16;
-            if (!take_rows(nl, s, cnt, lane, nkind, off, status)) continue;
-            set_rows(nl, i, cnt, lane, nkind, off);
-            if (lane == 0) *reinterpret_cast<double4 *>(nl.ref_xyz + 4 * (size_t)i) = pi;
-            if (nl.full_span != nullptr) {
-                jmin = __reduce_min_sync(0xffffffffu, jmin);
-                jmax = __reduce_max_sync(0xffffffffu, jmax);
-                if (lane == 0) {
-                    nl.full_span[2 * (size_t)i] = jmin;
-                    nl.full_span[2 * (size_t)i + 1] = jmax;
+            auto place = [&] {
+                int64_t off = 0;
+                cf = __reduce_add_sync(0xffffffffu, cf);
+                cs = __reduce_add_sync(0xffffffffu, cs);
+                const int cnt = lane == 0 ? cf & 0xffff : lane == 1 ? cf >> 16 : lane == 2 ? cs & 0xffff : cs >> 16;
+                if (!take_rows(nl, s, cnt, lane, nkind, off, status)) return false;
+                set_rows(nl, i, cnt, lane, nkind, off);
+                if (lane == 0) *reinterpret_cast<double4 *>(nl.ref_xyz + 4 * (size_t)i) = pi;
+                if (nl.full_span != nullptr) {
+                    jmin = __reduce_min_sync(0xffffffffu, jmin);
+                    jmax = __reduce_max_sync(0xffffffffu, jmax);
+                    if (lane == 0) {
+                        nl.full_span[2 * (size_t)i] = jmin;
+                        nl.full_span[2 * (size_t)i + 1] = jmax;
+                    }
                 }
-            }
-            wf = nl.full_cols + __shfl_sync(0xffffffffu, off, 0);
-            wh = nl.half_cols + __shfl_sync(0xffffffffu, off, 1);
-            if (shorts) {
-                wsf = nl.sfull_cols + __shfl_sync(0xffffffffu, off, 2);
-                wsh = nl.shalf_cols + __shfl_sync(0xffffffffu, off, 3);
-            }
-#pragma unroll 1
-            for (int b = 0; b < nch; b += step) {
-                if (step < NL_CHUNKS) n = stage(b, min(nch, b + step));
+                wf = nl.full_cols + __shfl_sync(0xffffffffu, off, 0);
+                wh = nl.half_cols + __shfl_sync(0xffffffffu, off, 1);
+                wsf = shorts ? nl.sfull_cols + __shfl_sync(0xffffffffu, off, 2) : nullptr;
+                wsh = shorts ? nl.shalf_cols + __shfl_sync(0xffffffffu, off, 3) : nullptr;
+                return true;
+            };
+            auto write = [&](int n) {
                 for (int t0 = 0; t0 < n; t0 += 32) {
                     const uint32_t st = t0 + lane < n ? W.stage[t0 + lane] : NL_DROPPED;
                     const bool v = st != NL_DROPPED;
@@ -570,7 +556,29 @@ nl_rows_kernel(const int32_t *__restrict__ atom_off, int nsys, int natoms, const
                         wsh += __popc(msh);
                     }
                 }
+                __syncwarp();  // the stage is the next part's
+            };
+            const int n = list(0, nch);
+            if (n > NL_STAGE) {
+                // too long for the stage: 32 chunks (1,024 candidates at most) at a
+                // time, once to be counted and again to be written.  48 chains of
+                // 4,962 atoms scaled to 0.9, where one row in six is that long:
+                // 2,719 us, 3,955 with FP64 scans of the 27 cells for those.
+                const int parts = (nch + 31) >> 5;
+#pragma unroll 1
+                for (int p = 0; p < 2 * parts; ++p) {
+                    if (p == parts && !place()) break;
+                    const int b = 32 * (p < parts ? p : p - parts);
+                    const int part = list(b, min(nch, b + 32));
+                    decide(part);
+                    if (p >= parts) write(part);
+                    __syncwarp();
+                }
+                continue;
             }
+            decide(n);
+            if (place()) write(n);
+            else __syncwarp();
         }
         __syncwarp();  // the masks and the stage are the next atoms'
     }
@@ -664,8 +672,8 @@ extern "C" int alma_nl_build(const AlmaBatch *b, const AlmaTopo *t, AlmaNL *nl, 
     const uint32_t *ew = t && t->excl_ptr ? t->excl_win : nullptr;
     // Two atoms per warp read each candidate once for both; below about two
     // waves of one-atom warps the chip has room for the shorter chains (16k
-    // atoms: 96 us with one, 97 with two; 24k: 160 and 152; 32k: 178 and 170; 65k:
-    // 492 and 438).
+    // atoms: 94 us with one, 95 with two; 24k: 157 and 150; 32k: 174 and 166; 65k:
+    // 481 and 431).
     auto rows = [&](auto kfn, int per_warp) {
         const int per_block = per_warp * NL_WARPS;
         kfn<<<(natoms + per_block - 1) / per_block, NL_WARPS * 32, 0, st>>>(
