@@ -53,8 +53,8 @@ C3_CHAINS, C3_PER_STEP, C2_PER_STEP = 256, 100, 1000
 L2_NOTE = "inputs larger than L2 (lists of 1.36 M atoms) and a 256 MiB L2 flush between GPU steps"
 # DRAM bytes (read + write) per proposal of the MC kernel, from one ncu capture
 # of a smaller case of the same workload, scaled by the proposals of a launch:
-# profiles/mc_kernel_batched_48_chains.md (168.8 MB / 266 proposals)
-DRAM_BYTES_PER_PROPOSAL = {"batched": 168.8e6 / 266}
+# profiles/mc_kernel_batched_48_chains.md (201.5 MB / 266 proposals)
+DRAM_BYTES_PER_PROPOSAL = {"batched": 201.5e6 / 266}
 
 
 def rank_info():
@@ -892,7 +892,8 @@ def run_profile_case(args):
     at the first drift flag); --config CL,NT[,K] picks the launch shape.
     "mc-batched": the first 48 chains of the batched workload (~0.25 M
     atoms), 20 warm-up proposals per chain, then one mc launch of up to 20
-    proposals per chain.  "forces": the single chain, one energy evaluation
+    proposals per chain, on the clusters and CTAs that the whole batch takes
+    (--config CL,NT for others).  "forces": the single chain, one energy evaluation
     and one alma_forces call (4 gradient kernels).  "energy": the first 48
     chains of the batched workload, one neighbor-list build, one full energy
     evaluation and one gradient (alma_forces).  The measured part sits
@@ -906,8 +907,8 @@ def run_profile_case(args):
         systems, _ = _our_systems(chains)
         batch = DeviceBatch(systems, precision="mixed")
         if args.profile == "mc-batched":
-            runner = MCRunner(batch, temps, seed=12345, policy=0, cluster_size=1, threads=args.threads,
-                              spec_teams=1)
+            cl, nt = (int(v) for v in (args.config or "4,0").split(",")[:2])
+            runner = MCRunner(batch, temps, seed=12345, policy=0, cluster_size=cl, threads=nt, spec_teams=1)
             runner.run(20)
             lim = int(runner.state()["step"].max()) + 20
             torch.cuda.synchronize()
