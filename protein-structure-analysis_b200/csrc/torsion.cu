@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(COMPOSE_THREADS) torsion_apply_kernel(ApplyArg
 // without any pays 4-5 us.  4,030 residues among 99 chains of 64: 2,761 us on
 // the one CTA of the mean (2,132 as one CTA of twice the threads, atoms apart),
 // 435 here; 1,000 among 40 of 64: 618 and 50.
-constexpr int LARGE_CTAS = 8, LARGE_CLUSTERS = 18;  // about a CTA per SM
+constexpr int LARGE_CTAS = 8, LARGE_CLUSTERS = 15;  // as many as fit at one CTA per SM
 
 __global__ void __launch_bounds__(COMPOSE_THREADS) torsion_apply_large_kernel(ApplyArgs A, int nsys, int limit) {
     __shared__ unsigned found[COMPOSE_THREADS / 32];
